@@ -189,7 +189,9 @@ static fg_status launch_splitk(fg_ctx* ctx, const TcMaps& maps, TcArgs& args, in
     const int splits = plan_splits(want, args.k_blocks, out_elems, sizeof(T), &kps);
     if (splits <= 1) return launch_any<Cfg>(ctx, maps, args, st);
     Scratch ws;
-    FG_TRY(ws.alloc(static_cast<size_t>(splits * out_elems) * sizeof(T), st));
+    // no room for the partial products: one split needs none
+    if (ws.alloc(static_cast<size_t>(splits * out_elems) * sizeof(T), st) != FG_OK)
+        return launch_any<Cfg>(ctx, maps, args, st);
     args.splits = splits;
     args.kb_per_split = kps;
     args.C = ws.p;
@@ -497,10 +499,18 @@ fg_status launch_split_bf16(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
         }
         return FG_OK;
     }
-    // Real-embedded sizes for complex: (M x 2K) * (2K x 2N).
+    if (cplx && (g.alpha_im != 0.0 || g.beta_im != 0.0))
+        return set_error(FG_ERR_UNSUPPORTED, "split CGEMM: complex alpha/beta must be real");
+    // Complex: the real GEMM (M x 2K) (2K x 2N), A and C the interleaved
+    // matrices as they lie, B embedded by the split pass; from here on it is
+    // dispatched like a real one (CTA pairs, split-K).
     const bool f16 = g.mode == FG_MODE_SPLIT_F16;  // two FP16 slices of scaled operands
     const int ns = (!f16 && g.slices == 3) ? 3 : 2;  // slices per operand
-    const long long M = g.M, K = cplx ? 2 * g.K : g.K, N = cplx ? 2 * g.N : g.N;
+    const int cw = cplx ? 2 : 1;
+    const long long M = g.M, K = cw * g.K, N = cw * g.N;
+    const long long lda = cw * g.lda, ldc = cw * g.ldc, a_ms = cw * g.a_mstride, c_ms = cw * g.c_stride;
+    const float* A = static_cast<const float*>(g.A);
+    const float* B = static_cast<const float*>(g.B);
     const long long pa = round_up(K, 8), pb = round_up(N, 8);  // bf16 elements, 16-byte pitch
     const size_t a_elems = static_cast<size_t>(pa * M * g.a_count);
     const size_t b_elems = static_cast<size_t>(pb * K * g.b_count);
@@ -516,82 +526,41 @@ fg_status launch_split_bf16(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
         amax = reinterpret_cast<unsigned*>(static_cast<uint8_t*>(s.p) + round_up(plane_bytes, 256));
         FG_CUDA(cudaMemsetAsync(amax, 0, 2 * sizeof(unsigned), st));
         // complex operands: max over the interleaved (re, im) floats
-        const int cw = cplx ? 2 : 1;
         const unsigned ga = static_cast<unsigned>(std::max<long long>(1, std::min<long long>(
-                                (g.M * g.K * cw * g.a_count / 4 + 255) / 256, 4LL * ctx->sm_count)));
+                                (M * K * g.a_count / 4 + 255) / 256, 4LL * ctx->sm_count)));
         const unsigned gb = static_cast<unsigned>(std::max<long long>(1, std::min<long long>(
-                                (g.K * g.N * cw * g.b_count / 4 + 255) / 256, 4LL * ctx->sm_count)));
-        if (g.M * g.K > 0)
-            amax_bits_kernel<<<ga, 256, 0, st>>>(static_cast<const float*>(g.A), g.M, g.K * cw, g.lda * cw,
-                                                 g.a_count, g.a_mstride * cw, amax);
-        if (g.K * g.N > 0)
-            amax_bits_kernel<<<gb, 256, 0, st>>>(static_cast<const float*>(g.B), g.K, g.N * cw, g.ldb * cw,
-                                                 g.b_count, g.b_mstride * cw, amax + 1);
+                                (g.K * N * g.b_count / 4 + 255) / 256, 4LL * ctx->sm_count)));
+        amax_bits_kernel<<<ga, 256, 0, st>>>(A, M, K, lda, g.a_count, a_ms, amax);
+        amax_bits_kernel<<<gb, 256, 0, st>>>(B, g.K, N, g.ldb * cw, g.b_count, g.b_mstride * cw, amax + 1);
         count_launch(2);
     }
-    if (cplx && f16) {
-        if (g.M * g.K > 0) {
-            split_f16_cplx_a_kernel<<<grid_for(g.M * g.K), 256, 0, st>>>(static_cast<const float2*>(g.A), g.M,
-                                                                         g.K, g.lda, ap, pa, amax);
-            count_launch();
-        }
-        if (g.K * g.N > 0) {
-            split_f16_cplx_b_kernel<<<grid_for(g.K * g.N), 256, 0, st>>>(static_cast<const float2*>(g.B), g.K,
-                                                                         g.N, g.ldb, bp, pb, amax + 1);
-            count_launch();
-        }
-    } else if (f16) {
-        ProfScope prof("split_f16", st);
-        if (M * K > 0) {
-            const dim3 grid(static_cast<unsigned>(std::min<long long>(M, 8LL * ctx->sm_count)), static_cast<unsigned>(g.a_count));
-            split_f16_kernel<<<grid, 256, 0, st>>>(static_cast<const float*>(g.A), M, K, g.lda, ap, pa, g.a_mstride,
-                                                   pa * M, amax);
-            count_launch();
-        }
-        if (K * N > 0) {
-            const dim3 grid(static_cast<unsigned>(std::min<long long>(K, 8LL * ctx->sm_count)), static_cast<unsigned>(g.b_count));
-            split_f16_kernel<<<grid, 256, 0, st>>>(static_cast<const float*>(g.B), K, N, g.ldb, bp, pb, g.b_mstride,
-                                                   pb * K, amax + 1);
-            count_launch();
-        }
-        prof.stop();
-    } else if (cplx) {
-        if (g.M * g.K > 0) {
-            if (ns == 3)
-                split_bf16_cplx_a_kernel<3><<<grid_for(g.M * g.K), 256, 0, st>>>(
-                    static_cast<const float2*>(g.A), g.M, g.K, g.lda, ap, pa);
+    {
+        ProfScope prof(f16 ? "split_f16" : "split_bf16", st);
+        const dim3 ga(static_cast<unsigned>(std::min<long long>(M, 8LL * ctx->sm_count)), static_cast<unsigned>(g.a_count));
+        const dim3 gb(static_cast<unsigned>(std::min<long long>(K, 8LL * ctx->sm_count)), static_cast<unsigned>(g.b_count));
+        if (f16)
+            split_f16_kernel<<<ga, 256, 0, st>>>(A, M, K, lda, ap, pa, a_ms, pa * M, amax);
+        else if (ns == 3)
+            split_bf16_kernel_t<3><<<ga, 256, 0, st>>>(A, M, K, lda, ap, pa, a_ms, pa * M);
+        else
+            split_bf16_kernel_t<2><<<ga, 256, 0, st>>>(A, M, K, lda, ap, pa, a_ms, pa * M);
+        if (cplx) {  // one matrix: complex batches were taken apart above
+            const unsigned gx = static_cast<unsigned>(
+                std::min<long long>((g.K * ((N + 7) / 8) + 255) / 256, 8LL * ctx->sm_count));
+            if (f16)
+                split_cplx_b_kernel<2, true><<<gx, 256, 0, st>>>(B, g.K, g.N, g.ldb, bp, pb, amax + 1);
+            else if (ns == 3)
+                split_cplx_b_kernel<3, false><<<gx, 256, 0, st>>>(B, g.K, g.N, g.ldb, bp, pb, nullptr);
             else
-                split_bf16_cplx_a_kernel<2><<<grid_for(g.M * g.K), 256, 0, st>>>(
-                    static_cast<const float2*>(g.A), g.M, g.K, g.lda, ap, pa);
-            count_launch();
+                split_cplx_b_kernel<2, false><<<gx, 256, 0, st>>>(B, g.K, g.N, g.ldb, bp, pb, nullptr);
+        } else if (f16) {
+            split_f16_kernel<<<gb, 256, 0, st>>>(B, K, N, g.ldb, bp, pb, g.b_mstride, pb * K, amax + 1);
+        } else if (ns == 3) {
+            split_bf16_kernel_t<3><<<gb, 256, 0, st>>>(B, K, N, g.ldb, bp, pb, g.b_mstride, pb * K);
+        } else {
+            split_bf16_kernel_t<2><<<gb, 256, 0, st>>>(B, K, N, g.ldb, bp, pb, g.b_mstride, pb * K);
         }
-        if (g.K * g.N > 0) {
-            if (ns == 3)
-                split_bf16_cplx_b_kernel<3><<<grid_for(g.K * g.N), 256, 0, st>>>(
-                    static_cast<const float2*>(g.B), g.K, g.N, g.ldb, bp, pb);
-            else
-                split_bf16_cplx_b_kernel<2><<<grid_for(g.K * g.N), 256, 0, st>>>(
-                    static_cast<const float2*>(g.B), g.K, g.N, g.ldb, bp, pb);
-            count_launch();
-        }
-    } else {
-        ProfScope prof("split_bf16", st);
-        if (M * K > 0) {
-            const dim3 grid(static_cast<unsigned>(std::min<long long>(M, 8LL * ctx->sm_count)), static_cast<unsigned>(g.a_count));
-            if (ns == 3)
-                split_bf16_kernel_t<3><<<grid, 256, 0, st>>>(static_cast<const float*>(g.A), M, K, g.lda, ap, pa, g.a_mstride, pa * M);
-            else
-                split_bf16_kernel_t<2><<<grid, 256, 0, st>>>(static_cast<const float*>(g.A), M, K, g.lda, ap, pa, g.a_mstride, pa * M);
-            count_launch();
-        }
-        if (K * N > 0) {
-            const dim3 grid(static_cast<unsigned>(std::min<long long>(K, 8LL * ctx->sm_count)), static_cast<unsigned>(g.b_count));
-            if (ns == 3)
-                split_bf16_kernel_t<3><<<grid, 256, 0, st>>>(static_cast<const float*>(g.B), K, N, g.ldb, bp, pb, g.b_mstride, pb * K);
-            else
-                split_bf16_kernel_t<2><<<grid, 256, 0, st>>>(static_cast<const float*>(g.B), K, N, g.ldb, bp, pb, g.b_mstride, pb * K);
-            count_launch();
-        }
+        count_launch(2);
         prof.stop();
     }
     FG_CUDA(cudaGetLastError());
@@ -611,16 +580,11 @@ fg_status launch_split_bf16(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
     args.tiles_n = static_cast<int>((N + CfgBf16x3::BN - 1) / CfgBf16x3::BN);
     args.k_blocks = static_cast<int>((K + CfgBf16x3::BK - 1) / CfgBf16x3::BK);
     args.C = g.C;
-    args.ldc = g.ldc;  // complex: in complex elements -> float pitch below
+    args.ldc = ldc;
     args.alpha = static_cast<float>(g.alpha_re);
     args.beta = static_cast<float>(g.beta_re);
     fill_batch(g, args);
-    if (cplx) {
-        if (g.alpha_im != 0.0 || g.beta_im != 0.0)
-            return set_error(FG_ERR_UNSUPPORTED, "split CGEMM: complex alpha/beta must be real");
-        args.cplx_half = static_cast<int>(g.N);
-        args.ldc = 2 * g.ldc;
-    }
+    args.strideC = c_ms;
     args.kchunk = split_kchunk();
     if (ns == 3) {
         // hi*hi + (hi*mid + mid*hi) + (hi*lo + lo*hi + mid*mid), smallest first
@@ -631,7 +595,7 @@ fg_status launch_split_bf16(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
         args.ops[4] = TcOp{0, 1, 1, 1, 1};
         args.ops[5] = TcOp{0, 0, 0, 1, 1};
         // the pair kernel where the tuned 3-product table picks a pair tile
-        if (!cplx && tune_lookup(TUNE_SPLIT_F32, M, N, K).variant == 2) {
+        if (tune_lookup(TUNE_SPLIT_F32, M, N, K).variant == 2) {
             args.tiles_m = static_cast<int>((M + CfgBf16x6Pair::BM - 1) / CfgBf16x6Pair::BM);
             args.tiles_n = static_cast<int>((N + CfgBf16x6Pair::BN - 1) / CfgBf16x6Pair::BN);
             return launch_pair<CfgBf16x6Pair>(ctx, maps, args, st);
@@ -642,23 +606,21 @@ fg_status launch_split_bf16(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
     args.ops[0] = TcOp{1, 0, 0, sf, sf};  // lo * hi
     args.ops[1] = TcOp{0, 1, 0, sf, sf};  // hi * lo
     args.ops[2] = TcOp{0, 0, 0, sf, sf};  // hi * hi
-    // Tuned tile variant / split-K (real products only; the complex
-    // embedding's interleaving epilogue runs unsplit with 128-wide tiles).
-    const TuneChoice c = cplx ? TuneChoice{0, 1} : tune_lookup(TUNE_SPLIT_F32, M, N, K);
+    const TuneChoice c = tune_lookup(TUNE_SPLIT_F32, M, N, K);  // tile variant and split-K
     float* C = static_cast<float*>(g.C);
     const float alpha = args.alpha, beta = args.beta;
     if (c.variant == 2) {
         args.tiles_m = static_cast<int>((M + CfgBf16x3Pair::BM - 1) / CfgBf16x3Pair::BM);
         args.tiles_n = static_cast<int>((N + CfgBf16x3Pair::BN - 1) / CfgBf16x3Pair::BN);
-        return launch_splitk<CfgBf16x3Pair, float>(ctx, maps, args, c.splits, C, g.ldc, g.c_stride,
+        return launch_splitk<CfgBf16x3Pair, float>(ctx, maps, args, c.splits, C, ldc, c_ms,
                                                    alpha, beta, 0, st);
     }
     if (c.variant == 1) {
         args.tiles_n = static_cast<int>((N + CfgBf16x3n64::BN - 1) / CfgBf16x3n64::BN);
-        return launch_splitk<CfgBf16x3n64, float>(ctx, maps, args, c.splits, C, g.ldc, g.c_stride,
+        return launch_splitk<CfgBf16x3n64, float>(ctx, maps, args, c.splits, C, ldc, c_ms,
                                                   alpha, beta, 0, st);
     }
-    return launch_splitk<CfgBf16x3, float>(ctx, maps, args, c.splits, C, g.ldc, g.c_stride, alpha,
+    return launch_splitk<CfgBf16x3, float>(ctx, maps, args, c.splits, C, ldc, c_ms, alpha,
                                            beta, 0, st);
 }
 

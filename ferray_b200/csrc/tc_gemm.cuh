@@ -10,7 +10,7 @@
 //   warps 2-5   epilogue: tcgen05.ld the accumulators of a finished tile
 //               (one TMEM lane = one output row per thread), combine them
 //               (wrapping i32, i16 byte-slice recombination, alpha/beta,
-//               quantized zero-point correction, complex interleave) and
+//               quantized zero-point correction) and
 //               store to global memory.
 // Accumulators live in TMEM and are double-buffered when they fit in the 512
 // columns, so the epilogue of tile t overlaps the MMAs of tile t+1.
@@ -97,7 +97,7 @@ struct TcArgs {
     // were formed from A 2^sA and B 2^sB (f16_scale_exp), so the epilogue
     // multiplies by 2^-sA 2^-sB.  Null: no scaling.
     const unsigned* f16_amax;
-    int cplx_half;             // EPI_F32: >0 writes column j<h as Re, j>=h as Im
+    int cplx_half;             // EPI_OZAKI: >0 writes column j<h as Re, j>=h as Im
     // EPI_QMM
     const int* row_sum;
     const int* col_sum;
@@ -389,32 +389,6 @@ __device__ __forceinline__ void epilogue_store(const TcArgs& p, int bz, int grow
         float* cbase = static_cast<float*>(p.C) + bz * p.strideC;
         // the FP16 split's operand scaling, undone (exact powers of two)
         const int unscale = p.f16_amax ? -(f16_scale_exp(p.f16_amax[0]) + f16_scale_exp(p.f16_amax[1])) : 0;
-        if (p.cplx_half > 0) {
-            // Column j of the real-embedded product is Re (j < h) or Im (j >= h)
-            // of complex column j mod h; C is interleaved (re, im).
-            const int h = p.cplx_half;
-            float* crow = cbase + (long long)grow * p.ldc;
-            float old[32];
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {  // loads first, then stores
-                const int col = gcol0 + j;
-                const int cc = col < h ? col : col - h;
-                old[j] = (p.beta != 0.f && j < ncols) ? crow[2 * cc + (col < h ? 0 : 1)] : 0.f;
-            }
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                if (j < ncols) {
-                    const int col = gcol0 + j;
-                    const int cc = col < h ? col : col - h;
-                    float acc = __uint_as_float(v[0][j]);
-                    if (unscale) acc = mul_pow2(acc, unscale);
-                    float o = p.alpha * acc;
-                    if (p.beta != 0.f) o = fmaf(p.beta, old[j], o);
-                    crow[2 * cc + (col < h ? 0 : 1)] = o;
-                }
-            }
-            return;
-        }
         float* crow = cbase + (long long)grow * p.ldc + gcol0;
         float out[32];
 #pragma unroll

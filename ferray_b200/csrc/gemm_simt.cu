@@ -8,6 +8,7 @@
 #include "tune.h"
 
 #include <algorithm>
+#include <cmath>
 #include <mutex>
 
 namespace fgrt {
@@ -113,74 +114,164 @@ static fg_status launch_dmma(fg_ctx* ctx, const Gemm& g, BatchMap bm, int splits
     return FG_OK;
 }
 
-// Plain SGEMM on the cp.async FFMA kernel (ffma_sgemm.cuh): A transposed
-// into packed scratch, B in place when aligned (else packed), same split-K
-// scheme.  Results are bit-identical to simt_gemm_real<float, 8, 8, 8>.
+// ---- plain SGEMM on the cp.async FFMA kernel (ffma_sgemm.cuh)
+//
+// Which tile and split-K count a shape takes.  The per-output order does not
+// depend on the tile, so this is about time alone; it is a model of the kernel
+// rather than a table by size bucket, because how full the last wave is
+// changes between two buckets.  A CTA alone on an SM runs at its latency-bound
+// rate, CTAs together share the SM's rate for that tile; the grid runs in
+// waves of occupancy x SMs, the last one spread evenly; two-warp CTAs fill the
+// four schedulers in pairs (an odd number of them takes the time of the next
+// even one); splits add the combine pass.  Rates and constants are a fit to
+// 1100 runs on a B200 (1.965 GHz; 7 tiles x 10 split counts over 21 shapes from
+// 256^3 to 4096^3 and 8 to 64 rows of 8192 x 8192): residual 7 %, and the
+// choice is within 6 % of the best of those runs for every shape, 1 % on
+// average.
+struct FfmaTileInfo {
+    int bm, bn, occ;
+    bool pairs;           // two-warp CTAs
+    double alone, most;   // GFLOP/s of an SM: one CTA, many
+};
+using FfmaT0 = FfmaTile<128, 128, 16, 8, 2, 0>;
+using FfmaT1 = FfmaTile<64, 128, 16, 8, 4, 0>;
+using FfmaT2 = FfmaTile<64, 64, 8, 8, 6, 4>;
+using FfmaT3 = FfmaTile<64, 64, 4, 8, 4, 4>;
+using FfmaT4 = FfmaTile<32, 128, 8, 8, 5, 4>;
+using FfmaT5 = FfmaTile<32, 64, 4, 8, 8, 4>;
+using FfmaT6 = FfmaTile<16, 128, 4, 8, 6, 0>;
+constexpr int FFMA_TILES = 7;
+constexpr FfmaTileInfo kFfmaTiles[FFMA_TILES] = {
+    {128, 128, 2, false, 425, 440}, {64, 128, 4, true, 230, 428}, {64, 64, 6, true, 220, 415},
+    {64, 64, 4, false, 308, 360},   {32, 128, 5, true, 185, 390}, {32, 64, 8, true, 185, 349},
+    {16, 128, 6, true, 185, 339},
+};
+
+struct FfmaChoice {
+    int tile, splits;
+    double us;
+};
+
+// fixed_splits > 0: that split count; only_tile >= 0: that tile.
+static FfmaChoice ffma_plan(int sms, long long M, long long N, long long K, long long batch, int fixed_splits,
+                            int only_tile) {
+    FfmaChoice best{std::max(only_tile, 0), std::max(fixed_splits, 1), 1e300};
+    const long long ku = (K + 63) / 64;
+    for (int s = fixed_splits > 0 ? fixed_splits : 1;; ++s) {
+        int kps = 0;
+        const int ns = plan_splits(s, static_cast<int>(ku), M * N * batch, sizeof(float), &kps);
+        if (ns == s || fixed_splits > 0) {
+            const double kk = static_cast<double>(std::min<long long>(K, 64LL * kps));
+            const double combine = ns > 1 ? 3.0 + (2.0 * ns + 1) * M * N * 4 * batch / 5.0e6 : 0.0;
+            for (int t = 0; t < FFMA_TILES; ++t) {
+                if (only_tile >= 0 && t != only_tile) continue;
+                const FfmaTileInfo& f = kFfmaTiles[t];
+                const double work = 2.0 * f.bm * f.bn * kk / 1e3;  // us at 1 GFLOP/s
+                auto dur = [&](long long c) {
+                    if (f.pairs) c = (c + 1) / 2 * 2;
+                    const double a = c * f.alone / f.most, a2 = a * a;
+                    const double rate = f.most * a / std::sqrt(std::sqrt(1.0 + a2 * a2));
+                    return c * work / rate + 0.3;
+                };
+                const long long units = (M + f.bm - 1) / f.bm * ((N + f.bn - 1) / f.bn) * ns * batch;
+                const long long slots = (long long)sms * f.occ, rem = units % slots;
+                double us = (units / slots) * dur(f.occ) + (rem ? dur((rem + sms - 1) / sms) : 0.0);
+                us = std::max(us, (M * K + K * N) * 4.0 * batch / 5.8e6) + 4.9 + combine;
+                if (us < best.us) best = FfmaChoice{t, ns, us};
+            }
+        }
+        if (fixed_splits > 0 || s >= TUNE_MAX_SPLITS || s >= ku) break;
+    }
+    return best;
+}
+
+// The packed transpose wants a K grid below 65536 blocks of 64, the kernel a
+// row grid below 65536 blocks of at least 16.
+constexpr long long kFfmaMaxK = 32LL * 65535;
+static bool ffma_ok(const Gemm& g) { return g.K <= kFfmaMaxK && g.M <= 16LL * 65535; }
+
+// One launch: At packed, B in place, into C or (splits > 1) into partials.
 template <class Cfg>
-static fg_status launch_ffma(const Gemm& g, int splits_want, cudaStream_t st) {
-    constexpr bool kSkinny = Cfg::BM == 32;
-    auto kern = kSkinny ? ffma_sgemm_skinny_kernel : ffma_sgemm_kernel;
+static fg_status launch_ffma_tile(const Gemm& g, const float* At, long long ldat, const BatchMap& bm, int splits,
+                                  int ksplit, float alpha, float beta, float* C, long long ldc, cudaStream_t st) {
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [kern] {
-        attr_err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    std::call_once(once, [] {
+        attr_err = cudaFuncSetAttribute(ffma_sgemm_kernel<Cfg>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         static_cast<int>(Cfg::SMEM));
     });
     FG_CUDA(attr_err);
+    dim3 grid(static_cast<unsigned>((g.N + Cfg::BN - 1) / Cfg::BN), static_cast<unsigned>((g.M + Cfg::BM - 1) / Cfg::BM),
+              static_cast<unsigned>(g.batch * splits));
+    ffma_sgemm_kernel<Cfg><<<grid, Cfg::THREADS, Cfg::SMEM, st>>>(
+        (int)g.M, (int)g.N, (int)g.K, alpha, At, ldat, static_cast<const float*>(g.B), g.ldb, beta, C, ldc, bm, g.batch,
+        ksplit);
+    count_launch();
+    FG_CUDA(cudaGetLastError());
+    return FG_OK;
+}
+
+template <class T>
+struct FfmaShifted;  // the same tile with B rows at any alignment
+template <int BM, int BN, int TM, int TN, int MINB, int BPAD>
+struct FfmaShifted<FfmaTile<BM, BN, TM, TN, MINB, BPAD, false>> {
+    using type = FfmaTile<BM, BN, TM, TN, MINB, BPAD, true>;
+};
+
+// A transposed into packed scratch, B in place, same split-K scheme as
+// launch_simt_real.  Results are bit-identical to simt_gemm_real<float, 8, 8, 8>
+// at equal split count.
+static fg_status launch_ffma(fg_ctx* ctx, const Gemm& g, int fixed_splits, int only_tile, cudaStream_t st) {
     const long long M = g.M, N = g.N, K = g.K;
-    const long long Mp = (M + 3) / 4 * 4, Np = (N + 3) / 4 * 4;
-    const float* A = static_cast<const float*>(g.A);
-    const float* B = static_cast<const float*>(g.B);
-    Scratch sa, sb;
+    const long long Mp = (M + 3) / 4 * 4;
+    const FfmaChoice c = ffma_plan(ctx->sm_count, M, N, K, g.batch, fixed_splits, only_tile);
+    const long long kunits = (K + 63) / 64;
+    int kps = static_cast<int>(kunits);
+    int splits = plan_splits(c.splits, static_cast<int>(kunits), M * N * g.batch, sizeof(float), &kps);
+    if ((long long)splits * g.batch > 65535) splits = 1;  // the grid's z extent
+    Scratch sa, ws;
     FG_TRY(sa.alloc(static_cast<size_t>(g.a_count * K * Mp) * sizeof(float), st));
     float* At = static_cast<float*>(sa.p);
-    transpose_pack_kernel<<<dim3(static_cast<unsigned>((Mp + 31) / 32), static_cast<unsigned>((K + 31) / 32),
+    transpose_pack_kernel<<<dim3(static_cast<unsigned>((Mp + 63) / 64), static_cast<unsigned>((K + 63) / 64),
                                  static_cast<unsigned>(g.a_count)),
-                            dim3(32, 8), 0, st>>>(A, (int)M, (int)K, g.lda, g.a_mstride, At, Mp);
+                            256, 0, st>>>(static_cast<const float*>(g.A), (int)M, (int)K, g.lda, g.a_mstride, At, Mp);
     count_launch();
-    const bool direct = (reinterpret_cast<uintptr_t>(B) % 16) == 0 && g.ldb % 4 == 0 && N % 4 == 0;
-    const float* Bk = B;
-    long long ldbk = g.ldb;
     BatchMap bm = batch_map(g);
     for (int d = 0; d < 4; ++d) bm.a_bstride[d] = g.a_istride[d] * K * Mp;
-    if (!direct) {
-        FG_TRY(sb.alloc(static_cast<size_t>(g.b_count * K * Np) * sizeof(float), st));
-        float* Bp = static_cast<float*>(sb.p);
-        pack_rows_kernel<<<dim3(static_cast<unsigned>(std::min<long long>((K * Np + 255) / 256, 4096)),
-                                static_cast<unsigned>(g.b_count)),
-                           256, 0, st>>>(B, (int)K, (int)N, g.ldb, g.b_mstride, Bp, Np);
-        count_launch();
-        Bk = Bp;
-        ldbk = Np;
-        for (int d = 0; d < 4; ++d) bm.b_bstride[d] = g.b_istride[d] * K * Np;
+    float* C = static_cast<float*>(g.C);
+    long long ldc = g.ldc;
+    float alpha = static_cast<float>(g.alpha_re), beta = static_cast<float>(g.beta_re);
+    // no room for the partial products: one split needs none
+    if (splits > 1 && ws.alloc(static_cast<size_t>(splits * M * N * g.batch) * sizeof(float), st) != FG_OK) splits = 1;
+    if (splits > 1) {
+        C = static_cast<float*>(ws.p);
+        ldc = N;
+        bm.c_bstride = M * N;
+        alpha = 1.f;
+        beta = 0.f;
     }
-    const int bcols = static_cast<int>(direct ? N : Np);
-    constexpr long long KUNIT = 64;
-    const long long kunits = (K + KUNIT - 1) / KUNIT;
-    int kps = static_cast<int>(kunits);
-    const int splits = plan_splits(splits_want, static_cast<int>(kunits), M * N * g.batch, sizeof(float), &kps);
-    if ((long long)splits * g.batch > 65535) return set_error(FG_ERR_UNSUPPORTED, "batch above 65535");
-    dim3 grid((N + Cfg::BN - 1) / Cfg::BN, (M + Cfg::BM - 1) / Cfg::BM, g.batch * splits);
-    if (splits <= 1) {
-        kern<<<grid, Cfg::THREADS, Cfg::SMEM, st>>>(
-            (int)M, (int)N, (int)K, (float)g.alpha_re, At, Mp, Bk, ldbk, bcols, (float)g.beta_re,
-            static_cast<float*>(g.C), g.ldc, bm, g.batch, (int)K);
-        count_launch();
-        FG_CUDA(cudaGetLastError());
-        return FG_OK;
+    const int ksplit = splits > 1 ? kps * 64 : static_cast<int>(K);
+    const bool aligned = (reinterpret_cast<uintptr_t>(g.B) & 15) == 0 && g.ldb % 4 == 0 &&
+                         (g.b_count == 1 || g.b_mstride % 4 == 0);
+    auto run = [&](auto tile) {
+        using T = decltype(tile);
+        if (aligned) return launch_ffma_tile<T>(g, At, Mp, bm, splits, ksplit, alpha, beta, C, ldc, st);
+        return launch_ffma_tile<typename FfmaShifted<T>::type>(g, At, Mp, bm, splits, ksplit, alpha, beta, C, ldc, st);
+    };
+    fg_status s = FG_OK;
+    switch (c.tile) {
+        case 0: s = run(FfmaT0{}); break;
+        case 1: s = run(FfmaT1{}); break;
+        case 2: s = run(FfmaT2{}); break;
+        case 3: s = run(FfmaT3{}); break;
+        case 4: s = run(FfmaT4{}); break;
+        case 5: s = run(FfmaT5{}); break;
+        default: s = run(FfmaT6{}); break;
     }
-    Scratch ws;
-    const long long out_elems = M * N * g.batch;
-    FG_TRY(ws.alloc(static_cast<size_t>(splits * out_elems) * sizeof(float), st));
-    BatchMap wbm = bm;
-    wbm.c_bstride = M * N;
-    kern<<<grid, Cfg::THREADS, Cfg::SMEM, st>>>(
-        (int)M, (int)N, (int)K, 1.f, At, Mp, Bk, ldbk, bcols, 0.f, static_cast<float*>(ws.p), N, wbm, g.batch,
-        (int)(kps * KUNIT));
-    splitk_reduce_kernel<float><<<grid_for(out_elems), 256, 0, st>>>(
-        static_cast<const float*>(ws.p), splits, M, N, g.batch, static_cast<float*>(g.C), g.ldc, g.c_stride,
-        (float)g.alpha_re, (float)g.beta_re, 0);
-    count_launch(2);
+    if (s != FG_OK || splits == 1) return s;
+    splitk_reduce_kernel<float><<<grid_for(M * N * g.batch), 256, 0, st>>>(
+        C, splits, M, N, g.batch, static_cast<float*>(g.C), g.ldc, g.c_stride, (float)g.alpha_re, (float)g.beta_re, 0);
+    count_launch();
     FG_CUDA(cudaGetLastError());
     return FG_OK;
 }
@@ -239,7 +330,7 @@ fg_status launch_simt(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
     if (g.dtype == FG_F64 || g.dtype == FG_F32) {  // profile under the tuned kernel's name
         const TuneChoice c = tune_lookup(g.dtype == FG_F64 ? TUNE_F64 : TUNE_F32, g.M, g.N, g.K);
         if (c.variant == 4) fam = g.dtype == FG_F64 ? "dmma_dgemm" : "ffma_sgemm";
-        if (c.variant == 5) fam = g.dtype == FG_F64 ? "dmma_dgemm_skinny" : "ffma_sgemm_skinny";
+        if (c.variant == 5) fam = g.dtype == FG_F64 ? "dmma_dgemm_skinny" : "ffma_sgemm";
     }
     ProfScope prof(fam, st);
     switch (g.dtype) {
@@ -256,18 +347,22 @@ fg_status launch_simt(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
         }
         case FG_F32: {
             const TuneChoice c = tune_lookup(TUNE_F32, g.M, g.N, g.K);
+            const bool forced = tune_forced(TUNE_F32);  // else ffma_plan's splits and tile
+            // Deep problems that the table (tuned with the slower kernel this
+            // family replaced) still gives a register-staged tile: 33 x 5675 x
+            // 1040 47 -> 35 us, 220 x 130 x 3365 29 -> 25 us; below K = 1024 the
+            // transpose launch costs more than it gives (279 x 195 x 802 17
+            // against 21 us).
+            if (!forced && c.variant < 4 && g.K > 1024 && g.batch == 1 && ffma_ok(g)) return launch_ffma(ctx, g, 0, -1, st);
             switch (c.variant) {
                 case 1: return launch_simt_real<float, 4, 4>(g, bm, c.splits, st);
                 case 2: return launch_simt_real<float, 2, 8>(g, bm, c.splits, st);
                 case 3: return launch_simt_real<float, 8, 2>(g, bm, c.splits, st);
                 case 4:
-                    // the packed transpose wants a K grid below 65536 blocks
-                    if (g.M > 0 && g.N > 0 && g.K > 0 && g.K <= 32LL * 65535)
-                        return launch_ffma<FfmaCfg>(g, c.splits, st);
+                    if (ffma_ok(g)) return launch_ffma(ctx, g, forced ? c.splits : 0, -1, st);
                     return launch_simt_real<float, 8, 8>(g, bm, c.splits, st);
                 case 5:
-                    if (g.M > 0 && g.N > 0 && g.K > 0 && g.K <= 32LL * 65535)
-                        return launch_ffma<FfmaSkinnyCfg>(g, c.splits, st);
+                    if (ffma_ok(g)) return launch_ffma(ctx, g, forced ? c.splits : 0, forced ? 4 : -1, st);
                     return launch_simt_real<float, 2, 8>(g, bm, c.splits, st);
                 default: return launch_simt_real<float, 8, 8>(g, bm, c.splits, st);
             }
@@ -307,7 +402,7 @@ fg_status launch_simt(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
             // GEMM (M x 2K) (2K x 2N) on it (same 8MNK flops, one FMA per
             // product); otherwise the 4M kernel.
             if (g.batch == 1 && g.alpha_im == 0.0 && g.beta_im == 0.0 && g.M > 0 && g.N > 0 && g.K > 0 &&
-                2 * g.K <= 32LL * 65535 && (reinterpret_cast<uintptr_t>(g.B) & 7) == 0) {
+                2 * g.K <= kFfmaMaxK && (reinterpret_cast<uintptr_t>(g.B) & 7) == 0) {
                 const TuneChoice c = tune_lookup(TUNE_F32, g.M, 2 * g.N, 2 * g.K);
                 if (c.variant == 4) {
                     Scratch bx;
@@ -323,7 +418,7 @@ fg_status launch_simt(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
                     r.B = bx.p;
                     r.ldb = 2 * g.N;
                     r.ldc = 2 * g.ldc;
-                    return launch_ffma<FfmaCfg>(r, c.splits, st);
+                    return launch_ffma(ctx, r, tune_forced(TUNE_F32) ? c.splits : 0, -1, st);
                 }
             }
             dim3 grid((g.N + 63) / 64, (g.M + 63) / 64, g.batch);

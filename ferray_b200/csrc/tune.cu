@@ -36,6 +36,10 @@ int tune_bucket(long long x) {
 
 int tune_variants(int op) { return (op >= 0 && op < TUNE_OPS) ? kVariants[op] : 0; }
 
+bool tune_forced(int op) {
+    return op >= 0 && op < TUNE_OPS && g_force_variant[op].load(std::memory_order_relaxed) >= 0;
+}
+
 TuneChoice tune_lookup(int op, long long m, long long n, long long k) {
     if (op < 0 || op >= TUNE_OPS) return {0, 1};
     const int fv = g_force_variant[op].load(std::memory_order_relaxed);

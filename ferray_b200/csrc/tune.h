@@ -30,6 +30,7 @@ struct TuneChoice {
 int tune_bucket(long long x);
 int tune_variants(int op);
 TuneChoice tune_lookup(int op, long long m, long long n, long long k);
+bool tune_forced(int op);  // a choice of fg_tune_force is in effect
 
 // Split count actually used: at most `want`, at most one split per K block,
 // no empty split, and a workspace (splits x out_elems x esize bytes) of at

@@ -5,6 +5,7 @@
 #include "simt_gemm.cuh"
 #include "dmma_gemm.cuh"
 #include "ffma_sgemm.cuh"
+#include "ffma_tile64.cuh"
 #include "tune.h"
 
 #include <algorithm>
@@ -276,6 +277,24 @@ static fg_status launch_ffma(fg_ctx* ctx, const Gemm& g, int fixed_splits, int o
     return FG_OK;
 }
 
+// Stacks of small problems: one CTA of 64 threads per 64 x 64 tile.
+static fg_status launch_tile64(const Gemm& g, const BatchMap& bm, cudaStream_t st) {
+    const long long tn = (g.N + 63) / 64, tm = (g.M + 63) / 64;
+    const Tile64Args a{(int)g.M, (int)g.N, (int)g.K, static_cast<const float*>(g.A), static_cast<const float*>(g.B),
+                       static_cast<float*>(g.C), g.lda, g.ldb, g.ldc, (float)g.alpha_re, (float)g.beta_re};
+    const bool vec = g.lda % 4 == 0 && g.ldb % 4 == 0 &&
+                     ((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B)) & 15) == 0 &&
+                     (g.a_count == 1 || g.a_mstride % 4 == 0) && (g.b_count == 1 || g.b_mstride % 4 == 0);
+    const dim3 grid(static_cast<unsigned>(g.batch), static_cast<unsigned>(tm * tn));
+    if (vec)
+        sgemm_tile64_kernel<true><<<grid, 64, 0, st>>>(a, bm, static_cast<int>(tn));
+    else
+        sgemm_tile64_kernel<false><<<grid, 64, 0, st>>>(a, bm, static_cast<int>(tn));
+    count_launch();
+    FG_CUDA(cudaGetLastError());
+    return FG_OK;
+}
+
 // Matrix-vector shapes (one operand is a vector; ferray's matmul of a 1-D
 // operand, products/mod.rs:362-437) go to the GEMV kernels.
 template <typename T>
@@ -348,6 +367,20 @@ fg_status launch_simt(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
         case FG_F32: {
             const TuneChoice c = tune_lookup(TUNE_F32, g.M, g.N, g.K);
             const bool forced = tune_forced(TUNE_F32);  // else ffma_plan's splits and tile
+            // Stacks.  Large matrices fill the GPU with the packed kernel's tiles
+            // (256^3 x 64: 55 against 58 us, 512^3 x 16: 97 against 109; 256 x 170
+            // x 240 x 106: 79 against 70); smaller ones take one CTA of 64 threads
+            // per tile (96 x 80 x 64 x 512: 22 us, 33 with the packed kernel, 47
+            // register-staged), unless there are fewer such CTAs than SMs, where
+            // 256 threads a tile have the shorter latency (191 x 37 x 44 x 32: 8.3
+            // against 5.9 us).
+            if (!forced && g.batch > 1) {
+                if (g.M * g.N * g.K >= (1LL << 24)) {
+                    if (ffma_ok(g)) return launch_ffma(ctx, g, 0, -1, st);
+                } else if ((g.M + 63) / 64 * ((g.N + 63) / 64) * g.batch > ctx->sm_count) {
+                    return launch_tile64(g, bm, st);
+                }
+            }
             // Deep problems that the table (tuned with the slower kernel this
             // family replaced) still gives a register-staged tile: 33 x 5675 x
             // 1040 47 -> 35 us, 220 x 130 x 3365 29 -> 25 us; below K = 1024 the

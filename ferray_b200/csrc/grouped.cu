@@ -73,7 +73,7 @@ struct fgrt::GroupedJob {
     long long arena = 0;
     int nseg = 0;
     int njobs = 0;  // prep launch blocks: segments cut at PREP_JOB_CHUNKS chunks
-    size_t sz_probs = 0, sz_maps = 0, sz_ptrs = 0, sz_segs = 0, sz_jobs = 0, sz_tiles = 0;
+    size_t sz_probs = 0, sz_maps = 0, sz_segs = 0, sz_jobs = 0, sz_tiles = 0;
     static constexpr size_t sz_sched = 256;  // the tile scheduler's counter
     // bound state
     void* dev = nullptr;
@@ -83,7 +83,7 @@ struct fgrt::GroupedJob {
     PrepSeg* d_segs = nullptr;
     PrepJob* d_jobs = nullptr;
     unsigned long long* d_counter = nullptr;
-    size_t host_bytes() const { return sz_probs + sz_maps + sz_ptrs + sz_segs + sz_jobs + sz_tiles + sz_sched; }
+    size_t host_bytes() const { return sz_probs + sz_maps + sz_segs + sz_jobs + sz_tiles + sz_sched; }
     size_t dev_bytes() const { return host_bytes() + static_cast<size_t>(arena); }
 };
 
@@ -146,17 +146,8 @@ fg_status grouped_job_build(fg_ctx* ctx, fg_dtype dtype, fg_mode mode, const fg_
         g.M = static_cast<int>(q.m);
         g.N = static_cast<int>(q.n);
         g.K = static_cast<int>(q.k);
-        // plain FP32: a 32 x 32 tile where it pads at most 0.7x the area a
-        // 64 x 64 one does (small problems; its FMAs cost more each)
-        int tb = bm;
-        if (j->kind == 0) {
-            const long long a64 = (q.m + 63) / 64 * 64 * ((q.n + 63) / 64 * 64);
-            const long long a32 = (q.m + 31) / 32 * 32 * ((q.n + 31) / 32 * 32);
-            if (10 * a32 <= 7 * a64) tb = 32;
-        }
-        g.tile = tb;
-        g.tiles_m = static_cast<int>((q.m + tb - 1) / tb);
-        g.tiles_n = static_cast<int>((q.n + tb - 1) / tb);
+        g.tiles_m = static_cast<int>((q.m + bm - 1) / bm);
+        g.tiles_n = static_cast<int>((q.n + bm - 1) / bm);
         g.tile_start = j->total_tiles;
         j->total_tiles += (long long)g.tiles_m * g.tiles_n;
         g.C = q.c;
@@ -209,9 +200,8 @@ fg_status grouped_job_build(fg_ctx* ctx, fg_dtype dtype, fg_mode mode, const fg_
     j->nseg = nseg;
     const int nmaps = j->kind == 2 ? 4 : 2;
     const size_t npp = static_cast<size_t>(std::max(np, 1));
-    j->sz_probs = rup(sizeof(GroupedProblem) * npp, 256);
+    j->sz_probs = rup((j->kind == 0 ? sizeof(SimtProblem) : sizeof(GroupedProblem)) * npp, 256);
     j->sz_maps = j->kind == 0 ? 0 : rup(sizeof(CUtensorMap) * nmaps * npp, 256);
-    j->sz_ptrs = j->kind == 0 ? rup((2 * sizeof(void*) + 2 * sizeof(long long)) * npp, 256) : 0;
     j->sz_segs = rup(sizeof(PrepSeg) * std::max(nseg, 1), 256);
     j->sz_jobs = rup(sizeof(PrepJob) * static_cast<size_t>(std::max(j->njobs, 1)), 256);
     j->sz_tiles = rup(sizeof(TileRec) * static_cast<size_t>(std::max<long long>(j->total_tiles, 1)), 256);
@@ -223,12 +213,21 @@ fg_status grouped_job_bind(GroupedJob* j, void* dev_base, void* host_stage) {
     const size_t npp = static_cast<size_t>(std::max(np, 1));
     char* dbase = static_cast<char*>(dev_base);
     char* hbase = static_cast<char*>(host_stage);
-    const size_t o_maps = j->sz_probs, o_ptrs = o_maps + j->sz_maps, o_segs = o_ptrs + j->sz_ptrs;
+    const size_t o_maps = j->sz_probs, o_segs = o_maps + j->sz_maps;
     const size_t o_jobs = o_segs + j->sz_segs, o_tiles = o_jobs + j->sz_jobs, o_sched = o_tiles + j->sz_tiles;
     char* d_arena = dbase + j->host_bytes();
     std::memset(hbase + o_sched, 0, j->sz_sched);
     j->d_counter = reinterpret_cast<unsigned long long*>(dbase + o_sched);
-    std::memcpy(hbase, j->probs.data(), sizeof(GroupedProblem) * np);
+    if (j->kind == 0) {
+        SimtProblem* hp = reinterpret_cast<SimtProblem*>(hbase);
+        for (int x = 0; x < np; ++x) {
+            const fg_problem& q = j->probs_in[x];
+            hp[x] = SimtProblem{static_cast<const float*>(q.a), static_cast<const float*>(q.b), static_cast<float*>(q.c),
+                                q.lda, q.ldb, q.ldc, j->probs[x].M, j->probs[x].N, j->probs[x].K, 0};
+        }
+    } else {
+        std::memcpy(hbase, j->probs.data(), sizeof(GroupedProblem) * np);
+    }
     TileRec* htiles = reinterpret_cast<TileRec*>(hbase + o_tiles);
     // Tiles of the deepest problems first: the scheduler hands them out in
     // this order, so the long tiles start first and the short ones fill in
@@ -238,10 +237,34 @@ fg_status grouped_job_bind(GroupedJob* j, void* dev_base, void* host_stage) {
     std::stable_sort(order.begin(), order.end(),
                      [&](int u, int v) { return j->probs[u].k_blocks > j->probs[v].k_blocks; });
     long long t = 0;
-    for (int x : order) {
-        const GroupedProblem& g = j->probs[x];
-        for (int tm = 0; tm < g.tiles_m; ++tm)
-            for (int tn = 0; tn < g.tiles_n; ++tn) htiles[t++] = TileRec{x, tm, tn, g.k_blocks};
+    if (j->kind == 0) {
+        // Within a factor of two of K, whole tiles first, then those with one
+        // half of the rows or columns: the CTAs of an SM then mostly run the
+        // same one of the kernel's four loops (mixed, they evict each other's
+        // instructions: 545 against 530 us for the 4096-problem batch), and the
+        // long tiles still start first.
+        for (size_t x0 = 0, x1; x0 < order.size(); x0 = x1) {
+            const int kb = j->probs[order[x0]].k_blocks;
+            for (x1 = x0; x1 < order.size() && 2 * j->probs[order[x1]].k_blocks > kb; ++x1) {
+            }
+            for (int type = 0; type < 4; ++type)
+                for (size_t i = x0; i < x1; ++i) {
+                    const int x = order[i];
+                    const GroupedProblem& g = j->probs[x];
+                    // rows / columns of tiles with both halves
+                    const int fm = std::min((g.M + 31) / 64, g.tiles_m), fn = std::min((g.N + 31) / 64, g.tiles_n);
+                    for (int tm = type & 2 ? fm : 0; tm < (type & 2 ? g.tiles_m : fm); ++tm)
+                        for (int tn = type & 1 ? fn : 0; tn < (type & 1 ? g.tiles_n : fn); ++tn)
+                            htiles[t++] = TileRec{x, tm, tn, g.k_blocks};
+                }
+        }
+        if (t != j->total_tiles) return set_error(FG_ERR_INVALID, "grouped plan: tile table mismatch");
+    } else {
+        for (int x : order) {
+            const GroupedProblem& g = j->probs[x];
+            for (int tm = 0; tm < g.tiles_m; ++tm)
+                for (int tn = 0; tn < g.tiles_n; ++tn) htiles[t++] = TileRec{x, tm, tn, g.k_blocks};
+        }
     }
     const TileRec* dtiles = reinterpret_cast<const TileRec*>(dbase + o_tiles);
     CUtensorMap* hmaps = reinterpret_cast<CUtensorMap*>(hbase + o_maps);
@@ -299,25 +322,9 @@ fg_status grouped_job_bind(GroupedJob* j, void* dev_base, void* host_stage) {
     }
     j->d_jobs = reinterpret_cast<PrepJob*>(dbase + o_jobs);
     if (j->kind == 0) {
-        const void** pa = reinterpret_cast<const void**>(hbase + o_ptrs);
-        const void** pb = pa + npp;
-        long long* la = reinterpret_cast<long long*>(pb + npp);
-        long long* lb = la + npp;
-        for (int x = 0; x < np; ++x) {
-            pa[x] = j->oa[x].src;
-            pb[x] = j->ob[x].src;
-            la[x] = j->oa[x].ld;
-            lb[x] = j->ob[x].ld;
-        }
-        const void** dpa = reinterpret_cast<const void**>(dbase + o_ptrs);
-        j->sargs.problems = reinterpret_cast<const GroupedProblem*>(dbase);
+        j->sargs.problems = reinterpret_cast<const SimtProblem*>(dbase);
         j->sargs.tiles = dtiles;
         j->sargs.tile_counter = j->d_counter;
-        j->sargs.a = dpa;
-        j->sargs.b = dpa + npp;
-        j->sargs.lda = reinterpret_cast<const long long*>(dpa + 2 * npp);
-        j->sargs.ldb = reinterpret_cast<const long long*>(dpa + 2 * npp) + npp;
-        j->sargs.count = np;
         j->sargs.total_tiles = j->total_tiles;
         j->sargs.alpha = 1.f;
         j->sargs.beta = 0.f;
@@ -380,7 +387,7 @@ static fg_status grouped_job_kernels(GroupedJob* j, cudaStream_t st) {
     FG_CUDA(cudaMemsetAsync(j->d_counter, 0, sizeof(unsigned long long), st));
     if (j->kind == 0) {
         ProfScope prof("simt_grouped_sgemm", st);
-        simt_grouped_sgemm<<<std::min<long long>(j->total_tiles, ctx->sm_count * 8), 128, 0, st>>>(j->sargs);
+        simt_grouped_sgemm<<<std::min<long long>(j->total_tiles, ctx->sm_count * 6), 64, 0, st>>>(j->sargs);
         prof.stop();
     } else if (j->kind == 1) {
         ProfScope prof("tc_grouped_i8", st);

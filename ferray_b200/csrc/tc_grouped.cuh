@@ -20,6 +20,7 @@
 // 8-row boxes spread over the accumulator's lane quadrants (spread_row), so
 // short tiles keep all four epilogue warps busy.
 #pragma once
+#include "ffma_tile64.cuh"
 #include "tc_gemm.cuh"
 
 namespace fg {
@@ -30,7 +31,6 @@ struct GroupedProblem {
     long long tile_start;  // first global tile of this problem
     void* C;
     long long ldc;         // elements
-    int tile;              // plain FP32 batches: square tile edge, 64 or 32
 };
 
 // Per global tile: problem index, tile row, tile column and the problem's K
@@ -589,180 +589,60 @@ static __global__ void __launch_bounds__(256) grouped_prep_kernel(const PrepSeg*
 }
 
 // ------------------------------------------------------------------ SIMT
-// Plain FP32 grouped GEMM (FFMA): 64x64 tiles, 128 threads, 4x8 outputs per
-// thread, persistent over the global tile list.
+// Plain FP32 grouped GEMM: CTAs of 64 threads walk the batch's 64 x 64 tiles
+// (ffma_tile64.cuh), handed out by an atomic counter, longest K first.  4096
+// problems with dims log-uniform in [8, 512] (14.4 GFLOP useful, 18.3 padded to
+// 32) take 485 us a call on a B200, against 769 with 128-thread tiles of scalar
+// FMAs padded to 64 (or 32 with 2 x 4 outputs a thread); 338 such problems 81
+// against 93.  What is left is the shared-memory / L1 pipe (79 % busy; FMA pipe
+// 59 %): 4-byte loads of rows at any alignment.
+struct SimtProblem {
+    const float* a;
+    const float* b;
+    float* c;
+    long long lda, ldb, ldc;
+    int m, n, k;
+    int pad;
+};
+
 struct SimtGroupedArgs {
-    const GroupedProblem* problems;
+    const SimtProblem* problems;
     const TileRec* tiles;  // [total_tiles]
     unsigned long long* tile_counter;  // next unclaimed tile (zeroed before the launch)
-    const void* const* a;  // per problem operand pointers and leading dims
-    const void* const* b;
-    const long long* lda;
-    const long long* ldb;
-    int count;
     long long total_tiles;
     float alpha, beta;
 };
 
-// A 32 x 32 tile of a small problem on the same 128 threads: 2 rows x 4
-// columns a thread, the same double-buffered K blocks of 16 and the same
-// per-output k order (one FMA per product, k ascending).  Uses the caller's
-// shared tiles (the first 32 columns of each row).
-__device__ __forceinline__ void grouped_tile32(const SimtGroupedArgs& g, const GroupedProblem& pr,
-                                               const float* __restrict__ A, const float* __restrict__ B,
-                                               long long lda, long long ldb, int m0, int n0,
-                                               float (*As)[16][68], float (*Bs)[16][68]) {
-    constexpr int BK = 16;
-    const int tid = threadIdx.x, tx = tid % 8, ty = tid / 8;
-    float ra[4], rb[4];
-    auto load = [&](int k0) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int e = tid + q * 128;  // 512 elements of each 32 x 16 / 16 x 32 tile
-            const int ar = e / BK, ac = e % BK;
-            const int gr = m0 + ar, gk = k0 + ac;
-            ra[q] = (gr < pr.M && gk < pr.K) ? A[(long long)gr * lda + gk] : 0.f;
-            const int br = e / 32, bc = e % 32;
-            const int gk2 = k0 + br, gn = n0 + bc;
-            rb[q] = (gk2 < pr.K && gn < pr.N) ? B[(long long)gk2 * ldb + gn] : 0.f;
-        }
-    };
-    auto store = [&](int buf) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int e = tid + q * 128;
-            As[buf][e % BK][e / BK] = ra[q];
-            Bs[buf][e / 32][e % 32] = rb[q];
-        }
-    };
-    float acc[2][4] = {};
-    const int kblocks = (pr.K + BK - 1) / BK;
-    load(0);
-    __syncthreads();  // the previous tile's readers are done with buffer 0
-    store(0);
-    __syncthreads();
-    for (int kb = 0; kb < kblocks; ++kb) {
-        const int cur = kb & 1;
-        if (kb + 1 < kblocks) load((kb + 1) * BK);
-#pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            const float2 a2 = *reinterpret_cast<const float2*>(&As[cur][kk][ty * 2]);
-            const float4 b4 = *reinterpret_cast<const float4*>(&Bs[cur][kk][tx * 4]);
-            const float af[2] = {a2.x, a2.y}, bf[4] = {b4.x, b4.y, b4.z, b4.w};
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(af[i], bf[j], acc[i][j]);
-        }
-        if (kb + 1 < kblocks) store(cur ^ 1);
+static __global__ void __launch_bounds__(64, 6) simt_grouped_sgemm(const SimtGroupedArgs g) {
+    __shared__ Tile64Smem s;
+    // The first tile of a CTA is its block index; the next one is claimed before
+    // the last K block of the current one (claimed a tile ahead, the heaviest
+    // tiles would be dealt out in pairs: 338 problems took 171 us a call, 81 so), its record
+    // loaded before the stores, so both arrive behind work.
+    __shared__ TileRec rec;
+    __shared__ int more;
+    if (static_cast<long long>(blockIdx.x) >= g.total_tiles) return;
+    TileRec tr = g.tiles[blockIdx.x];
+    long long t = 0;
+    for (;;) {
+        const SimtProblem r = g.problems[tr.problem];
+        const int m0 = tr.tm * 64, n0 = tr.tn * 64;
+        sgemm_tile64<false>(
+            Tile64Args{min(r.m - m0, 64), min(r.n - n0, 64), r.k, r.a + m0 * r.lda, r.b + n0, r.c + m0 * r.ldc + n0, r.lda,
+                       r.ldb, r.ldc, g.alpha, g.beta},
+            0, 0, s,
+            [&] {
+                if (threadIdx.x == 0) t = gridDim.x + static_cast<long long>(atomicAdd(g.tile_counter, 1ull));
+            },
+            [&] {
+                if (threadIdx.x == 0) {
+                    more = t < g.total_tiles;
+                    if (t < g.total_tiles) rec = g.tiles[t];
+                }
+            });
         __syncthreads();
-    }
-    float* C = static_cast<float*>(pr.C);
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int gr = m0 + ty * 2 + i;
-        if (gr >= pr.M) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int gc = n0 + tx * 4 + j;
-            if (gc >= pr.N) continue;
-            float* p = C + (long long)gr * pr.ldc + gc;
-            float o = g.alpha * acc[i][j];
-            if (g.beta != 0.f) o = fmaf(g.beta, *p, o);
-            *p = o;
-        }
-    }
-}
-
-static __global__ void __launch_bounds__(128) simt_grouped_sgemm(const SimtGroupedArgs g) {
-    constexpr int BM = 64, BN = 64, BK = 16, NT = 128;
-    constexpr int PER = BM * BK / NT;  // elements of each operand a thread loads per K block
-    __shared__ __align__(16) float As[2][BK][BM + 4];
-    __shared__ __align__(16) float Bs[2][BK][BN + 4];
-    // 16 x 8 threads, 4 rows x 8 columns each (two 4-column groups 32 apart)
-    const int tid = threadIdx.x, tx = tid % 8, ty = tid / 8;
-    // device-side tile scheduler: thread 0 claims the next tile for the CTA;
-    // two slots, so the claim for tile i + 1 cannot overwrite the index
-    // others may still be reading for tile i
-    __shared__ long long claim[2];
-    for (int i = 0;; ++i) {
-        if (tid == 0) claim[i & 1] = static_cast<long long>(atomicAdd(g.tile_counter, 1ull));
-        __syncthreads();
-        const long long t = claim[i & 1];
-        if (t >= g.total_tiles) break;
-        const TileRec tr = g.tiles[t];
-        const int pi = tr.problem;
-        const GroupedProblem pr = g.problems[pi];
-        const float* A = static_cast<const float*>(g.a[pi]);
-        const float* B = static_cast<const float*>(g.b[pi]);
-        const long long lda = g.lda[pi], ldb = g.ldb[pi];
-        if (pr.tile == 32) {
-            grouped_tile32(g, pr, A, B, lda, ldb, tr.tm * 32, tr.tn * 32, As, Bs);
-            continue;
-        }
-        const int m0 = tr.tm * BM, n0 = tr.tn * BN;
-        // Next K block into registers while this one is computed; shared
-        // tiles double-buffered, one barrier per K block.
-        float ra[PER], rb[PER];
-        auto load = [&](int k0) {
-#pragma unroll
-            for (int q = 0; q < PER; ++q) {
-                const int e = tid + q * NT;
-                const int ar = e / BK, ac = e % BK;
-                const int gr = m0 + ar, gk = k0 + ac;
-                ra[q] = (gr < pr.M && gk < pr.K) ? A[(long long)gr * lda + gk] : 0.f;
-                const int br = e / BN, bc = e % BN;
-                const int gk2 = k0 + br, gn = n0 + bc;
-                rb[q] = (gk2 < pr.K && gn < pr.N) ? B[(long long)gk2 * ldb + gn] : 0.f;
-            }
-        };
-        auto store = [&](int buf) {
-#pragma unroll
-            for (int q = 0; q < PER; ++q) {
-                const int e = tid + q * NT;
-                As[buf][e % BK][e / BK] = ra[q];
-                Bs[buf][e / BN][e % BN] = rb[q];
-            }
-        };
-        float acc[4][8] = {};
-        const int kblocks = (pr.K + BK - 1) / BK;
-        load(0);
-        __syncthreads();  // the previous tile's readers are done with buffer 0
-        store(0);
-        __syncthreads();
-        for (int kb = 0; kb < kblocks; ++kb) {
-            const int cur = kb & 1;
-            if (kb + 1 < kblocks) load((kb + 1) * BK);
-#pragma unroll
-            for (int kk = 0; kk < BK; ++kk) {
-                const float4 a4 = *reinterpret_cast<const float4*>(&As[cur][kk][ty * 4]);
-                const float4 b0 = *reinterpret_cast<const float4*>(&Bs[cur][kk][tx * 4]);
-                const float4 b1 = *reinterpret_cast<const float4*>(&Bs[cur][kk][32 + tx * 4]);
-                const float af[4] = {a4.x, a4.y, a4.z, a4.w};
-                const float bf[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(af[i], bf[j], acc[i][j]);
-            }
-            if (kb + 1 < kblocks) store(cur ^ 1);
-            __syncthreads();
-        }
-        float* C = static_cast<float*>(pr.C);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int gr = m0 + ty * 4 + i;
-            if (gr >= pr.M) continue;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int gc = n0 + (j / 4) * 32 + tx * 4 + (j % 4);
-                if (gc >= pr.N) continue;
-                float* p = C + (long long)gr * pr.ldc + gc;
-                float o = g.alpha * acc[i][j];
-                if (g.beta != 0.f) o = fmaf(g.beta, *p, o);
-                *p = o;
-            }
-        }
+        if (!more) break;
+        tr = rec;  // rewritten only after the next tile's barriers
     }
 }
 

@@ -63,7 +63,7 @@ static EncodeTiledFn encode_fn() {
 }
 
 fg_status encode_map(CUtensorMap* map, CUtensorMapDataType dt, int rank, const void* base,
-                     const uint64_t* dims, const uint64_t* strides_bytes, const uint32_t* box) {
+                     const uint64_t* dims, const uint64_t* strides_bytes, const uint32_t* box, bool swizzle) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return set_error(FG_ERR_DEVICE, "cuTensorMapEncodeTiled unavailable");
     cuuint32_t estr[3] = {1, 1, 1};
@@ -71,7 +71,7 @@ fg_status encode_map(CUtensorMap* map, CUtensorMapDataType dt, int rank, const v
                     reinterpret_cast<const cuuint64_t*>(dims),
                     reinterpret_cast<const cuuint64_t*>(strides_bytes),
                     reinterpret_cast<const cuuint32_t*>(box), estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS)
         return set_error(FG_ERR_INVALID, "cuTensorMapEncodeTiled failed (code " + std::to_string((int)r) + ")");

@@ -63,9 +63,8 @@ static fg_status launch_simt_real(const Gemm& g, BatchMap bm, int splits_want, c
     simt_gemm_real<T, 8, TMM, TNN><<<grid, 256, 0, st>>>((int)g.M, (int)g.N, (int)g.K, T(1), A, g.lda, B,
                                                    g.ldb, T(0), static_cast<T*>(ws.p), g.N, wbm,
                                                    g.batch, (int)(kps * KUNIT));
-    splitk_reduce_kernel<T><<<grid_for(out_elems), 256, 0, st>>>(
-        static_cast<const T*>(ws.p), splits, g.M, g.N, g.batch, static_cast<T*>(g.C), g.ldc,
-        g.c_stride, (T)g.alpha_re, (T)g.beta_re, 0);
+    splitk_reduce<T>(static_cast<const T*>(ws.p), splits, g.M, g.N, g.batch, static_cast<T*>(g.C), g.ldc,
+        g.c_stride, (T)g.alpha_re, (T)g.beta_re, 0, st);
     count_launch(2);
     FG_CUDA(cudaGetLastError());
     return FG_OK;
@@ -107,9 +106,8 @@ static fg_status launch_dmma(fg_ctx* ctx, const Gemm& g, BatchMap bm, int splits
     dmma_gemm_f64_kernel<Cfg><<<grid, Cfg::THREADS, Cfg::SMEM, st>>>(
         (int)g.M, (int)g.N, (int)g.K, 1.0, A, g.lda, B, g.ldb, 0.0, static_cast<double*>(ws.p), g.N, wbm,
         g.batch, (int)(kps * KUNIT));
-    splitk_reduce_kernel<double><<<grid_for(out_elems), 256, 0, st>>>(
-        static_cast<const double*>(ws.p), splits, g.M, g.N, g.batch, static_cast<double*>(g.C), g.ldc,
-        g.c_stride, g.alpha_re, g.beta_re, 0);
+    splitk_reduce<double>(static_cast<const double*>(ws.p), splits, g.M, g.N, g.batch, static_cast<double*>(g.C), g.ldc,
+        g.c_stride, g.alpha_re, g.beta_re, 0, st);
     count_launch(2);
     FG_CUDA(cudaGetLastError());
     return FG_OK;
@@ -270,8 +268,7 @@ static fg_status launch_ffma(fg_ctx* ctx, const Gemm& g, int fixed_splits, int o
         default: s = run(FfmaT6{}); break;
     }
     if (s != FG_OK || splits == 1) return s;
-    splitk_reduce_kernel<float><<<grid_for(M * N * g.batch), 256, 0, st>>>(
-        C, splits, M, N, g.batch, static_cast<float*>(g.C), g.ldc, g.c_stride, (float)g.alpha_re, (float)g.beta_re, 0);
+    splitk_reduce<float>(C, splits, M, N, g.batch, static_cast<float*>(g.C), g.ldc, g.c_stride, (float)g.alpha_re, (float)g.beta_re, 0, st);
     count_launch();
     FG_CUDA(cudaGetLastError());
     return FG_OK;
@@ -330,8 +327,8 @@ static fg_status launch_gemv(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
     FG_TRY(ws.alloc(static_cast<size_t>(splits * g.N) * sizeof(T), st));
     gemv_cols_kernel<T><<<grid, 256, 0, st>>>((int)g.N, (int)g.K, ksplit, (T)g.alpha_re, A, 1, B, g.ldb,
                                               (T)g.beta_re, static_cast<T*>(ws.p), g.N);
-    splitk_reduce_kernel<T><<<grid_for(g.N), 256, 0, st>>>(static_cast<const T*>(ws.p), splits, 1, g.N, 1,
-                                                           C, g.ldc, 0, (T)g.alpha_re, (T)g.beta_re, 0);
+    splitk_reduce<T>(static_cast<const T*>(ws.p), splits, 1, g.N, 1,
+                                                           C, g.ldc, 0, (T)g.alpha_re, (T)g.beta_re, 0, st);
     count_launch(2);
     FG_CUDA(cudaGetLastError());
     return FG_OK;

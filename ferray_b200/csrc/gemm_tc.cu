@@ -14,6 +14,7 @@
 #include "runtime.h"
 #include "tc_gemm.cuh"
 #include "tc_gemm2.cuh"
+#include "tc_rows.cuh"
 #include "tune.h"
 
 namespace fgrt {
@@ -178,7 +179,7 @@ static fg_status launch_any(fg_ctx* ctx, const TcMaps& maps, TcArgs& args, cudaS
 
 // Launches Cfg with up to `want` K splits (tuned).  With more than one
 // split the kernel writes dense partial products [split][batch][M][N] into a
-// workspace and splitk_reduce_kernel combines them into C (wrapping int32
+// workspace and splitk_reduce combines them into C (wrapping int32
 // sum + accumulate, or alpha * sum + beta * C).
 template <class Cfg, typename T>
 static fg_status launch_splitk(fg_ctx* ctx, const TcMaps& maps, TcArgs& args, int want, T* C,
@@ -201,9 +202,8 @@ static fg_status launch_splitk(fg_ctx* ctx, const TcMaps& maps, TcArgs& args, in
     args.alpha = 1.f;
     args.beta = 0.f;
     FG_TRY(launch_any<Cfg>(ctx, maps, args, st));
-    splitk_reduce_kernel<T><<<grid_for_total(out_elems), 256, 0, st>>>(
-        static_cast<const T*>(ws.p), splits, M, N, args.batch, C, ldc, strideC, alpha, beta,
-        accumulate);
+    splitk_reduce<T>(static_cast<const T*>(ws.p), splits, M, N, args.batch, C, ldc, strideC, alpha, beta,
+        accumulate, st);
     count_launch();
     FG_CUDA(cudaGetLastError());
     return FG_OK;
@@ -474,6 +474,94 @@ fg_status launch_half_tc(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
                                          st);
 }
 
+// Few rows: the split SGEMM that cuts B into slices on the way to the tensor
+// core (tc_rows.cuh).  A's planes come from the usual pass (small here).
+template <int MP, bool TMA>
+static fg_status launch_rows(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
+    using Cfg = TcRowsCfg<MP, TMA>;
+    static std::once_flag once;
+    static cudaError_t attr_err = cudaSuccess;
+    std::call_once(once, [] {
+        attr_err = cudaFuncSetAttribute(tc_rows_kernel<Cfg>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        static_cast<int>(tc_rows_smem_bytes<Cfg>()));
+    });
+    FG_CUDA(attr_err);
+    const long long M = g.M, N = g.N, K = g.K, pa = round_up(K, 8);
+    const int tiles = static_cast<int>((N + Cfg::BN - 1) / Cfg::BN);
+    const int k_blocks = static_cast<int>((K + Cfg::BK - 1) / Cfg::BK);
+    // Split K so that the units fill whole waves of one CTA per SM: a K block
+    // (64 x 128 of B) takes an SM about 0.75 us at the HBM rate, a combine pass
+    // about 3 us and its bytes.
+    int want = 1;
+    double best = 1e300;
+    for (int c = 1; c <= TUNE_MAX_SPLITS; ++c) {
+        int kps = 0;
+        if (plan_splits(c, k_blocks, M * N, sizeof(float), &kps) != c) continue;
+        const long long waves = ((long long)tiles * c + ctx->sm_count - 1) / ctx->sm_count;
+        const double us = 0.75 * waves * kps + (c > 1 ? 3.0 + (2.0 * c + 1) * M * N * 4 / 5.0e6 : 0.0);
+        if (us < best) best = us, want = c;
+    }
+    int kps = k_blocks;
+    int splits = plan_splits(want, k_blocks, M * N, sizeof(float), &kps);
+    Scratch sp, ws;
+    FG_TRY(sp.alloc(static_cast<size_t>(2 * pa * M) * sizeof(__nv_bfloat16), st));
+    if (splits > 1 && ws.alloc(static_cast<size_t>(splits * M * N) * sizeof(float), st) != FG_OK) {
+        splits = 1;  // no room for the partial products
+        kps = k_blocks;
+    }
+    BfPlanes ap{};
+    ap.p[0] = static_cast<__nv_bfloat16*>(sp.p);
+    ap.p[1] = ap.p[0] + pa * M;
+    const unsigned ga = static_cast<unsigned>(
+        std::min<long long>((M * (pa / 8) + 255) / 256, 8LL * ctx->sm_count));
+    split_bf16_kernel_t<2><<<ga, 256, 0, st>>>(static_cast<const float*>(g.A), M, K, g.lda, ap, pa, 0, 0);
+    count_launch();
+    CUtensorMap hi, lo;
+    int r3;
+    FG_TRY(operand_map(&hi, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, ap.p[0], K, M, pa * 2, 1, 0, 64, MP, &r3));
+    FG_TRY(operand_map(&lo, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, ap.p[1], K, M, pa * 2, 1, 0, 64, MP, &r3));
+    CUtensorMap mb{};
+    if (TMA) {
+        const uint64_t dims[2] = {static_cast<uint64_t>(N), static_cast<uint64_t>(K)};
+        const uint64_t strides[1] = {static_cast<uint64_t>(g.ldb) * 4};
+        const uint32_t box[2] = {Cfg::BN, Cfg::BK};
+        FG_TRY(encode_map(&mb, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, g.B, dims, strides, box, false));
+    }
+    TcRowsArgs a{};
+    a.B = static_cast<const float*>(g.B);
+    a.ldb = g.ldb;
+    a.M = static_cast<int>(M);
+    a.N = static_cast<int>(N);
+    a.K = static_cast<int>(K);
+    a.tiles = tiles;
+    a.splits = splits;
+    a.k_blocks = k_blocks;
+    a.kb_per_split = kps;
+    a.kchunk = std::max(split_kchunk(), 1);
+    a.C = splits > 1 ? static_cast<float*>(ws.p) : static_cast<float*>(g.C);
+    a.ldc = splits > 1 ? N : g.ldc;
+    a.split_stride = splits > 1 ? M * N : 0;
+    a.alpha = splits > 1 ? 1.f : static_cast<float>(g.alpha_re);
+    a.beta = splits > 1 ? 0.f : static_cast<float>(g.beta_re);
+    a.status = ctx->d_status;
+    a.timeout_ns = kTimeoutNs;
+    const int grid = static_cast<int>(std::min<long long>((long long)tiles * splits, ctx->sm_count));
+    {
+        ProfScope prof("tc_rows_3xbf16", st);
+        tc_rows_kernel<Cfg><<<grid, Cfg::THREADS, tc_rows_smem_bytes<Cfg>(), st>>>(hi, lo, mb, a);
+        prof.stop();
+    }
+    count_launch();
+    FG_CUDA(cudaGetLastError());
+    if (splits > 1) {
+        splitk_reduce<float>(a.C, splits, M, N, 1, static_cast<float*>(g.C), g.ldc, 0, static_cast<float>(g.alpha_re),
+            static_cast<float>(g.beta_re), 0, st);
+        count_launch();
+        FG_CUDA(cudaGetLastError());
+    }
+    return FG_OK;
+}
+
 // 3xBF16: C = alpha * (Alo*Bhi + Ahi*Blo + Ahi*Bhi) + beta * C, f32 accumulate.
 fg_status launch_split_bf16(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
     const bool cplx = g.dtype == FG_C32;
@@ -506,6 +594,15 @@ fg_status launch_split_bf16(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
     // dispatched like a real one (CTA pairs, split-K).
     const bool f16 = g.mode == FG_MODE_SPLIT_F16;  // two FP16 slices of scaled operands
     const int ns = (!f16 && g.slices == 3) ? 3 : 2;  // slices per operand
+    // Up to 64 rows B is read once, so cutting it in a pass of its own triples the
+    // bytes: a call with 32 x 8192 x 8192 takes 64 us by the rows kernel against
+    // 156, 64 x 64 x 64 12.3 against 14.5 (36 shapes of 1-64 rows: 1.14-2.7x).
+    if (!cplx && !f16 && ns == 2 && g.batch == 1 && g.M <= 64 && !tune_forced(TUNE_SPLIT_F32)) {
+        const bool tma = tma_ok(g.B, g.ldb * 4, 1, 0);
+        if (g.M <= 16) return tma ? launch_rows<16, true>(ctx, g, st) : launch_rows<16, false>(ctx, g, st);
+        if (g.M <= 32) return tma ? launch_rows<32, true>(ctx, g, st) : launch_rows<32, false>(ctx, g, st);
+        return tma ? launch_rows<64, true>(ctx, g, st) : launch_rows<64, false>(ctx, g, st);
+    }
     const int cw = cplx ? 2 : 1;
     const long long M = g.M, K = cw * g.K, N = cw * g.N;
     const long long lda = cw * g.lda, ldc = cw * g.ldc, a_ms = cw * g.a_mstride, c_ms = cw * g.c_stride;

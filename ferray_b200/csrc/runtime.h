@@ -177,8 +177,9 @@ fg_status grouped_job_bind(GroupedJob* j, void* dev_base, void* host_stage);
 fg_status grouped_job_launch(GroupedJob* j, cudaStream_t st);
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no
-// link-time dependency on libcuda).
+// link-time dependency on libcuda).  swizzle: 128-byte (the operand tiles of
+// tcgen05.mma), else rows as they lie.
 fg_status encode_map(CUtensorMap* map, CUtensorMapDataType dt, int rank, const void* base,
-                     const uint64_t* dims, const uint64_t* strides_bytes, const uint32_t* box);
+                     const uint64_t* dims, const uint64_t* strides_bytes, const uint32_t* box, bool swizzle = true);
 
 }  // namespace fgrt

@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 8 && TMM == 8 && TNN == 8) 
 // x = A[0, :]; a block owns 32 x G columns (16-byte loads along N), its 8
 // warps take interleaved K rows and are summed in shared memory in warp
 // order; blockIdx.y splits K (partials to a workspace, combined by
-// splitk_reduce_kernel) when the columns alone do not fill the GPU.
+// splitk_reduce) when the columns alone do not fill the GPU.
 template <typename T>
 __global__ void __launch_bounds__(256)
     gemv_rows_kernel(int M, int K, T alpha, const T* __restrict__ A, long long lda,

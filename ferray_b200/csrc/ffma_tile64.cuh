@@ -38,11 +38,41 @@ struct Tile64Args {
     float alpha, beta;
 };
 
+// Sums of the closed accumulators of a tile, each thread its own.
+struct Tile64Totals {
+    float4 x[16][64];
+};
+
+// Adds the accumulators to the totals (sets them the first time) and clears
+// them, or on the last call leaves the sum in them.
+template <int RH, int CH>
+__device__ __forceinline__ void tile64_fold(uint64_t (&acc)[8][4], Tile64Totals& tot, bool first, bool more) {
+#pragma unroll
+    for (int i = 0; i < RH * 4; ++i)
+#pragma unroll
+        for (int h = 0; h < CH; ++h) {
+            float4& t = tot.x[i * 2 + h][threadIdx.x];
+            const float2 u = unpack2(acc[i][2 * h]), w = unpack2(acc[i][2 * h + 1]);
+            float4 v = make_float4(u.x, u.y, w.x, w.y);
+            if (!first) {
+                const float4 o = t;
+                v = make_float4(o.x + v.x, o.y + v.y, o.z + v.z, o.w + v.w);
+            }
+            if (more) {
+                t = v;
+                acc[i][2 * h] = acc[i][2 * h + 1] = 0;
+            } else {
+                acc[i][2 * h] = pack2(v.x, v.y);
+                acc[i][2 * h + 1] = pack2(v.z, v.w);
+            }
+        }
+}
+
 // acc over all of K for RH row halves and CH column halves.  VEC: rows of A and
 // B are 16-byte aligned; A comes in 16-byte loads, B by 16-byte cp.async.
-template <int RH, int CH, bool VEC, class Last>
+template <int RH, int CH, bool VEC, bool FOLD, class Last>
 __device__ __forceinline__ void tile64_loop(const Tile64Args& p, int m0, int n0, Tile64Smem& s,
-                                            uint64_t (&acc)[8][4], Last last) {
+                                            uint64_t (&acc)[8][4], Last last, Tile64Totals* tot, int chain) {
     constexpr int BK = 16, T = 64, U = 8;
     const int tid = threadIdx.x, tx = tid % 8, ty = tid / 8;
     // A, 4-byte: 8 k of 8 rows per step of 64 threads, the two k halves of the
@@ -178,13 +208,18 @@ __device__ __forceinline__ void tile64_loop(const Tile64Args& p, int m0, int n0,
             store(cur ^ 1);
             __syncthreads();
         }
+        if constexpr (FOLD) {
+            if ((kb + 1) % chain == 0 || kb + 1 == kblocks) tile64_fold<RH, CH>(acc, *tot, kb < chain, kb + 1 < kblocks);
+        }
     }
 }
 
 // C tile (m0, n0) = alpha A B + beta C.  All 64 threads of the CTA.  `last` runs
 // before the last K block is computed, `done` between the K loop and the stores.
-template <bool VEC, class Last, class Done>
-__device__ __forceinline__ void sgemm_tile64(const Tile64Args& p, int m0, int n0, Tile64Smem& s, Last last, Done done) {
+// FOLD: an accumulator is closed every `chain` K blocks.
+template <bool VEC, bool FOLD, class Last, class Done>
+__device__ __forceinline__ void sgemm_tile64(const Tile64Args& p, int m0, int n0, Tile64Smem& s, Last last, Done done,
+                                             Tile64Totals* tot = nullptr, int chain = 0) {
     uint64_t acc[8][4];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
@@ -192,13 +227,13 @@ __device__ __forceinline__ void sgemm_tile64(const Tile64Args& p, int m0, int n0
         for (int j = 0; j < 4; ++j) acc[i][j] = 0;
     const bool r2 = p.M - m0 > 32, c2 = p.N - n0 > 32;
     if (r2 && c2)
-        tile64_loop<2, 2, VEC>(p, m0, n0, s, acc, last);
+        tile64_loop<2, 2, VEC, FOLD>(p, m0, n0, s, acc, last, tot, chain);
     else if (r2)
-        tile64_loop<2, 1, VEC>(p, m0, n0, s, acc, last);
+        tile64_loop<2, 1, VEC, FOLD>(p, m0, n0, s, acc, last, tot, chain);
     else if (c2)
-        tile64_loop<1, 2, VEC>(p, m0, n0, s, acc, last);
+        tile64_loop<1, 2, VEC, FOLD>(p, m0, n0, s, acc, last, tot, chain);
     else
-        tile64_loop<1, 1, VEC>(p, m0, n0, s, acc, last);
+        tile64_loop<1, 1, VEC, FOLD>(p, m0, n0, s, acc, last, tot, chain);
     done();
     const int tx = threadIdx.x % 8, ty = threadIdx.x / 8;
     const bool vec = p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
@@ -233,14 +268,16 @@ __device__ __forceinline__ void sgemm_tile64(const Tile64Args& p, int m0, int n0
 // on the same tile of different problems, so on the same one of the four
 // loops.
 template <bool VEC>
-static __global__ void __launch_bounds__(64, 6) sgemm_tile64_kernel(Tile64Args p, BatchMap bm, int tiles_n) {
+static __global__ void __launch_bounds__(64, 6)
+    sgemm_tile64_kernel(Tile64Args p, BatchMap bm, int tiles_n, int chain) {
     __shared__ Tile64Smem s;
+    __shared__ Tile64Totals tot;
     long long oa, ob;
     batch_offsets(bm, blockIdx.x, oa, ob);
     p.A += oa;
     p.B += ob;
     p.C += blockIdx.x * bm.c_bstride;
-    sgemm_tile64<VEC>(p, blockIdx.y / tiles_n * 64, blockIdx.y % tiles_n * 64, s, [] {}, [] {});
+    sgemm_tile64<VEC, true>(p, blockIdx.y / tiles_n * 64, blockIdx.y % tiles_n * 64, s, [] {}, [] {}, &tot, chain);
 }
 
 }  // namespace fg

@@ -146,20 +146,30 @@ constexpr FfmaTileInfo kFfmaTiles[FFMA_TILES] = {
     {16, 128, 6, true, 185, 339},
 };
 
+// K units of 64 per accumulator when the shape is split `want` ways.
+static int chain_units(const Gemm& g, int want) {
+    int kps = 0;
+    plan_splits(want, static_cast<int>((g.K + 63) / 64), g.M * g.N * g.batch, sizeof(float), &kps);
+    return kps;
+}
+
 struct FfmaChoice {
     int tile, splits;
     double us;
 };
 
-// fixed_splits > 0: that split count; only_tile >= 0: that tile.
+// fixed_splits > 0: that split count; only_tile >= 0: that tile.  max_chain: the
+// longest run of k that one accumulator may take (64-deep units): the size
+// table's split count also bounds the rounding error, which grows with the square
+// root of that run, so the model may split further than the table, never less.
 static FfmaChoice ffma_plan(int sms, long long M, long long N, long long K, long long batch, int fixed_splits,
-                            int only_tile) {
+                            int only_tile, int max_chain) {
     FfmaChoice best{std::max(only_tile, 0), std::max(fixed_splits, 1), 1e300};
     const long long ku = (K + 63) / 64;
     for (int s = fixed_splits > 0 ? fixed_splits : 1;; ++s) {
         int kps = 0;
         const int ns = plan_splits(s, static_cast<int>(ku), M * N * batch, sizeof(float), &kps);
-        if (ns == s || fixed_splits > 0) {
+        if (fixed_splits > 0 || (ns == s && (kps <= max_chain || s == TUNE_MAX_SPLITS))) {
             const double kk = static_cast<double>(std::min<long long>(K, 64LL * kps));
             const double combine = ns > 1 ? 3.0 + (2.0 * ns + 1) * M * N * 4 * batch / 5.0e6 : 0.0;
             for (int t = 0; t < FFMA_TILES; ++t) {
@@ -220,10 +230,12 @@ struct FfmaShifted<FfmaTile<BM, BN, TM, TN, MINB, BPAD, false>> {
 // A transposed into packed scratch, B in place, same split-K scheme as
 // launch_simt_real.  Results are bit-identical to simt_gemm_real<float, 8, 8, 8>
 // at equal split count.
-static fg_status launch_ffma(fg_ctx* ctx, const Gemm& g, int fixed_splits, int only_tile, cudaStream_t st) {
+// `table`: the tuned choice for the shape (its split count fixed when forced).
+static fg_status launch_ffma(fg_ctx* ctx, const Gemm& g, TuneChoice table, int only_tile, cudaStream_t st) {
     const long long M = g.M, N = g.N, K = g.K;
     const long long Mp = (M + 3) / 4 * 4;
-    const FfmaChoice c = ffma_plan(ctx->sm_count, M, N, K, g.batch, fixed_splits, only_tile);
+    const FfmaChoice c = ffma_plan(ctx->sm_count, M, N, K, g.batch, tune_forced(TUNE_F32) ? table.splits : 0, only_tile,
+                                   chain_units(g, table.splits));
     const long long kunits = (K + 63) / 64;
     int kps = static_cast<int>(kunits);
     int splits = plan_splits(c.splits, static_cast<int>(kunits), M * N * g.batch, sizeof(float), &kps);
@@ -274,19 +286,32 @@ static fg_status launch_ffma(fg_ctx* ctx, const Gemm& g, int fixed_splits, int o
     return FG_OK;
 }
 
-// Stacks of small problems: one CTA of 64 threads per 64 x 64 tile.
-static fg_status launch_tile64(const Gemm& g, const BatchMap& bm, cudaStream_t st) {
+// Time of a stack by launch_tile64: a 16-deep K block takes 2.25 us with six CTAs
+// on an SM, 1 us alone, less where tiles have half the rows or columns (fit to
+// 512^3 x 16, 256^3 x 64, 1024 x 1024 x 256 x 4 and 300 x 700 x 2000 x 3, within 16 %).
+static double tile64_us(int sms, const Gemm& g) {
+    const long long tm = (g.M + 63) / 64, tn = (g.N + 63) / 64, units = tm * tn * g.batch, slots = 6LL * sms;
+    const double whole = static_cast<double>((g.M + 31) / 32 * ((g.N + 31) / 32)) / (4 * tm * tn);
+    const long long last = (units % slots + sms - 1) / sms;
+    return 4.9 + (g.K + 15) / 16 * whole * (2.25 * (units / slots) + (last ? 0.75 + 0.25 * last : 0.0));
+}
+
+// Stacks of small problems: one CTA of 64 threads per 64 x 64 tile.  Where the
+// tuned table splits K (the shape's latency, for one matrix), the kernel closes an
+// accumulator at the same places, so the rounding stays that of the split.
+static fg_status launch_tile64(const Gemm& g, const BatchMap& bm, TuneChoice table, cudaStream_t st) {
     const long long tn = (g.N + 63) / 64, tm = (g.M + 63) / 64;
     const Tile64Args a{(int)g.M, (int)g.N, (int)g.K, static_cast<const float*>(g.A), static_cast<const float*>(g.B),
                        static_cast<float*>(g.C), g.lda, g.ldb, g.ldc, (float)g.alpha_re, (float)g.beta_re};
+    const int chain = 4 * chain_units(g, table.splits);  // 16-deep K blocks
     const bool vec = g.lda % 4 == 0 && g.ldb % 4 == 0 &&
                      ((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B)) & 15) == 0 &&
                      (g.a_count == 1 || g.a_mstride % 4 == 0) && (g.b_count == 1 || g.b_mstride % 4 == 0);
     const dim3 grid(static_cast<unsigned>(g.batch), static_cast<unsigned>(tm * tn));
     if (vec)
-        sgemm_tile64_kernel<true><<<grid, 64, 0, st>>>(a, bm, static_cast<int>(tn));
+        sgemm_tile64_kernel<true><<<grid, 64, 0, st>>>(a, bm, static_cast<int>(tn), chain);
     else
-        sgemm_tile64_kernel<false><<<grid, 64, 0, st>>>(a, bm, static_cast<int>(tn));
+        sgemm_tile64_kernel<false><<<grid, 64, 0, st>>>(a, bm, static_cast<int>(tn), chain);
     count_launch();
     FG_CUDA(cudaGetLastError());
     return FG_OK;
@@ -364,35 +389,31 @@ fg_status launch_simt(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
         case FG_F32: {
             const TuneChoice c = tune_lookup(TUNE_F32, g.M, g.N, g.K);
             const bool forced = tune_forced(TUNE_F32);  // else ffma_plan's splits and tile
-            // Stacks.  Large matrices fill the GPU with the packed kernel's tiles
-            // (256^3 x 64: 55 against 58 us, 512^3 x 16: 97 against 109; 256 x 170
-            // x 240 x 106: 79 against 70); smaller ones take one CTA of 64 threads
-            // per tile (96 x 80 x 64 x 512: 22 us, 33 with the packed kernel, 47
-            // register-staged), unless there are fewer such CTAs than SMs, where
-            // 256 threads a tile have the shorter latency (191 x 37 x 44 x 32: 8.3
-            // against 5.9 us).
-            if (!forced && g.batch > 1) {
-                if (g.M * g.N * g.K >= (1LL << 24)) {
-                    if (ffma_ok(g)) return launch_ffma(ctx, g, 0, -1, st);
-                } else if ((g.M + 63) / 64 * ((g.N + 63) / 64) * g.batch > ctx->sm_count) {
-                    return launch_tile64(g, bm, st);
-                }
+            // Stacks: one CTA of 64 threads per tile or the packed kernel,
+            // whichever its model puts first (96 x 80 x 64 x 512: 22 us against 33,
+            // 47 register-staged; 300 x 700 x 2000 x 3: 135 against 70), unless there
+            // are fewer tiles than SMs, where 256 threads a tile have the shorter
+            // latency (191 x 37 x 44 x 32: 5.9 us, 8.3 with 64).
+            if (!forced && g.batch > 1 && (g.M + 63) / 64 * ((g.N + 63) / 64) * g.batch > ctx->sm_count) {
+                const double packed = 4.0 + ffma_plan(ctx->sm_count, g.M, g.N, g.K, g.batch, 0, -1, chain_units(g, c.splits)).us;
+                if (!ffma_ok(g) || tile64_us(ctx->sm_count, g) < packed) return launch_tile64(g, bm, c, st);
+                return launch_ffma(ctx, g, c, -1, st);
             }
             // Deep problems that the table (tuned with the slower kernel this
             // family replaced) still gives a register-staged tile: 33 x 5675 x
             // 1040 47 -> 35 us, 220 x 130 x 3365 29 -> 25 us; below K = 1024 the
             // transpose launch costs more than it gives (279 x 195 x 802 17
             // against 21 us).
-            if (!forced && c.variant < 4 && g.K > 1024 && g.batch == 1 && ffma_ok(g)) return launch_ffma(ctx, g, 0, -1, st);
+            if (!forced && c.variant < 4 && g.K > 1024 && g.batch == 1 && ffma_ok(g)) return launch_ffma(ctx, g, c, -1, st);
             switch (c.variant) {
                 case 1: return launch_simt_real<float, 4, 4>(g, bm, c.splits, st);
                 case 2: return launch_simt_real<float, 2, 8>(g, bm, c.splits, st);
                 case 3: return launch_simt_real<float, 8, 2>(g, bm, c.splits, st);
                 case 4:
-                    if (ffma_ok(g)) return launch_ffma(ctx, g, forced ? c.splits : 0, -1, st);
+                    if (ffma_ok(g)) return launch_ffma(ctx, g, c, -1, st);
                     return launch_simt_real<float, 8, 8>(g, bm, c.splits, st);
                 case 5:
-                    if (ffma_ok(g)) return launch_ffma(ctx, g, forced ? c.splits : 0, forced ? 4 : -1, st);
+                    if (ffma_ok(g)) return launch_ffma(ctx, g, c, forced ? 4 : -1, st);
                     return launch_simt_real<float, 2, 8>(g, bm, c.splits, st);
                 default: return launch_simt_real<float, 8, 8>(g, bm, c.splits, st);
             }
@@ -448,7 +469,7 @@ fg_status launch_simt(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
                     r.B = bx.p;
                     r.ldb = 2 * g.N;
                     r.ldc = 2 * g.ldc;
-                    return launch_ffma(ctx, r, tune_forced(TUNE_F32) ? c.splits : 0, -1, st);
+                    return launch_ffma(ctx, r, c, -1, st);
                 }
             }
             dim3 grid((g.N + 63) / 64, (g.M + 63) / 64, g.batch);

@@ -627,7 +627,7 @@ static __global__ void __launch_bounds__(64, 6) simt_grouped_sgemm(const SimtGro
     for (;;) {
         const SimtProblem r = g.problems[tr.problem];
         const int m0 = tr.tm * 64, n0 = tr.tn * 64;
-        sgemm_tile64<false>(
+        sgemm_tile64<false, false>(
             Tile64Args{min(r.m - m0, 64), min(r.n - n0, 64), r.k, r.a + m0 * r.lda, r.b + n0, r.c + m0 * r.ldc + n0, r.lda,
                        r.ldb, r.ldc, g.alpha, g.beta},
             0, 0, s,

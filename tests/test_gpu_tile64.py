@@ -57,3 +57,20 @@ def test_ragged_edges(fg):
     fg.gemm_grouped(problems)
     for a, b, c in arrays:
         np.testing.assert_array_equal(c.to_numpy(), _reference(fg, a, b))
+
+
+@pytest.mark.parametrize("m,n,k", [(23, 29, 240), (64, 64, 500), (33, 97, 1000), (70, 20, 2000)])
+def test_stack_keeps_the_split_rounding(fg, m, n, k):
+    """Where the table splits K, the stack kernel closes its accumulators at the
+    same places and adds them in the same order: same bits as the split form."""
+    batch = 160
+    _, splits = fg.tune_lookup("f32", m, n, k)
+    assert splits > 1
+    r = np.random.default_rng(k)
+    a = r.standard_normal((batch, m, k)).astype(np.float32)
+    b = r.standard_normal((batch, k, n)).astype(np.float32)
+    da, db = fg.DeviceArray.from_numpy(a), fg.DeviceArray.from_numpy(b)
+    got = fg.matmul(da, db).to_numpy()
+    with fg.tune_forced("f32", 0, splits):
+        want = fg.matmul(da, db).to_numpy()
+    np.testing.assert_array_equal(got, want)

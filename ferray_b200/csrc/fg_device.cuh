@@ -23,6 +23,8 @@ struct DevStatus {
     int where;      // which wait gave up (role * 16 + site)
     int block;      // blockIdx.x of the first failure
     int pad;
+    int* host_flag; // pinned host word set along with code: fg_sync reads that
+                    // instead of copying this struct back after every wait
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -39,6 +41,8 @@ __device__ __forceinline__ void report_error(DevStatus* st, int code, int where)
     if (st != nullptr && atomicCAS(&st->code, 0, code) == 0) {
         st->where = where;
         st->block = blockIdx.x;
+        __threadfence_system();
+        if (st->host_flag) *static_cast<volatile int*>(st->host_flag) = 1;
     }
 }
 

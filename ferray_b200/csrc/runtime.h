@@ -23,6 +23,7 @@ struct fg_ctx {
     // copies of one row panel overlap the GEMM of another
     cudaStream_t pipe_comp = nullptr, pipe_out = nullptr;
     fg::DevStatus* d_status = nullptr;  // kernel error word (device)
+    int* h_flag = nullptr;              // pinned, mapped: nonzero once a kernel wrote it
     std::mutex mu;
     std::mutex host_mu;  // one pipelined host-pointer call at a time
 };

@@ -25,8 +25,9 @@ using namespace fg;
 // 6 stages, for problems with few output tiles.
 using CfgI8 = TcCfg<KIND_I8, 256, 4, 1, 1, 1, 1, EPI_I32>;
 using CfgI8n128 = TcCfg<KIND_I8, 128, 6, 1, 1, 1, 1, EPI_I32>;
-// 256 x 256 tiles on CTA pairs (cta_group::2), 6 stages of 32 KB per CTA.
-using CfgI8Pair = Tc2Cfg<KIND_I8, 256, 7, 1, 1, 1, 1, EPI_I32>;
+// 256 x 256 tiles on CTA pairs (cta_group::2), 6 stages of 32 KB per CTA (7 would
+// fit without the epilogue's staging memory, and gain nothing).
+using CfgI8Pair = Tc2Cfg<KIND_I8, 256, 6, 1, 1, 1, 1, EPI_I32>;
 // 256 x 512 tiles on CTA pairs: one A tile feeds two N = 256 MMAs into two
 // TMEM accumulators (all 512 columns, single-buffered); 4 stages of 48 KB.
 using CfgI8PairW = Tc2Cfg<KIND_I8, 256, 4, 1, 2, 2, 2, EPI_I32, 0, 1>;
@@ -41,9 +42,11 @@ using CfgBf16x3n64 = TcCfg<KIND_BF16, 64, 4, 2, 2, 1, 3, EPI_F32, 1>;
 // 256 x 128 tiles on CTA pairs, 4 stages of 48 KB per CTA.
 using CfgBf16x3Pair = Tc2Cfg<KIND_BF16, 128, 4, 2, 2, 1, 3, EPI_F32, 1>;
 // bf16 / f16 operands as given (one product): 128 x 128 single-CTA tiles with
-// 6 stages of 32 KB, or 256 x 128 CTA-pair tiles with 8 stages of 24 KB per CTA.
+// 6 stages of 32 KB, 256 x 128 CTA-pair tiles with 8 stages of 24 KB per CTA, or
+// (half_wide below) 256 x 256 CTA-pair tiles with 6 stages of 32 KB per CTA.
 using CfgHalf = TcCfg<KIND_BF16, 128, 6, 1, 1, 1, 1, EPI_F32, 1>;
 using CfgHalfPair = Tc2Cfg<KIND_BF16, 128, 8, 1, 1, 1, 1, EPI_F32, 1>;
+using CfgHalfPairW = Tc2Cfg<KIND_BF16, 256, 6, 1, 1, 1, 1, EPI_F32, 1>;
 // 6 products (3 slices) on CTA pairs: 256 x 128 tiles, 3 stages of 72 KB per
 // CTA, hi*hi and the corrections in two TMEM accumulators.
 using CfgBf16x6Pair = Tc2Cfg<KIND_BF16, 128, 3, 3, 3, 2, 6, EPI_F32, 1>;
@@ -431,6 +434,22 @@ fg_status launch_qmm(fg_ctx* ctx, long long M, long long N, long long K, const u
     return launch_cfg<CfgQmm>(ctx, maps, args, st);
 }
 
+// 256 x 256 instead of 256 x 128 tiles for a 16-bit product on CTA pairs?  A wide
+// tile stages a third fewer bytes per MAC (the narrow one is bound by its shared-
+// memory traffic) but a wave of them lasts about 1.75 narrow waves, so it pays
+// where it saves enough waves.  Narrow / wide, B200, us: 8192^3 902 / 758, 4096^3
+// 119 / 112, 3072^3 55 / 50, 512 x 8192 x 8192 68 / 58 (4 waves against 7 or
+// better); 2560^3 37 / 42, 2304^3 34 / 38, 1536^3 14.3 / 19.5, 2816 x 5632 x 1408
+// 49 / 52 (more).  At 4 against 7 the short runs lose (4096 x 4096 x 1024 39 / 41)
+// and the long ones gain (K >= 2048).  K splits are tuned for the narrow tile.
+static bool half_wide(const fg_ctx* ctx, const Gemm& g, int splits) {
+    if (splits > 1) return false;
+    const long long pairs = ctx->sm_count / 2, rows = (g.M + 255) / 256 * g.batch;
+    const long long wide = (rows * ((g.N + 255) / 256) + pairs - 1) / pairs;
+    const long long narrow = (rows * ((g.N + 127) / 128) + pairs - 1) / pairs;
+    return 7 * wide < 4 * narrow || (7 * wide == 4 * narrow && g.K >= 2048);
+}
+
 // bf16 x bf16 / f16 x f16 -> f32 straight from the caller's 16-bit operands
 // (gemm/mod.rs:851-933 widen them to f32 for an SGEMM): one tcgen05 kind::f16
 // product per K block, K accumulated in TMEM chunks summed in FP32
@@ -463,6 +482,12 @@ fg_status launch_half_tc(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
     args.ops[0] = TcOp{0, 0, 0, fmt, fmt};
     float* C = static_cast<float*>(g.C);
     const TuneChoice c = tune_lookup(TUNE_SPLIT_F32, g.M, g.N, g.K);
+    if (c.variant == 2 && half_wide(ctx, g, c.splits)) {
+        args.tiles_m = static_cast<int>((g.M + CfgHalfPairW::BM - 1) / CfgHalfPairW::BM);
+        args.tiles_n = static_cast<int>((g.N + CfgHalfPairW::BN - 1) / CfgHalfPairW::BN);
+        return launch_splitk<CfgHalfPairW, float>(ctx, maps, args, c.splits, C, g.ldc, g.c_stride, 1.f,
+                                                  args.beta, 0, st);
+    }
     if (c.variant == 2) {
         args.tiles_m = static_cast<int>((g.M + CfgHalfPair::BM - 1) / CfgHalfPair::BM);
         args.tiles_n = static_cast<int>((g.N + CfgHalfPair::BN - 1) / CfgHalfPair::BN);

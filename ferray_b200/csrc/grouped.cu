@@ -39,7 +39,7 @@ fg_status set_smem_attr() {
     static cudaError_t err = cudaSuccess;
     std::call_once(once, [] {
         err = cudaFuncSetAttribute(tc_grouped_kernel<Cfg>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(tc_smem_bytes<Cfg>()));
+                                   static_cast<int>(tc_smem_bytes<Cfg, false>()));
     });
     if (err != cudaSuccess) return fgrt::cuda_error(err, "cudaFuncSetAttribute(grouped)");
     return FG_OK;
@@ -391,11 +391,11 @@ static fg_status grouped_job_kernels(GroupedJob* j, cudaStream_t st) {
         prof.stop();
     } else if (j->kind == 1) {
         ProfScope prof("tc_grouped_i8", st);
-        tc_grouped_kernel<CfgGroupedI8><<<grid, CfgGroupedI8::THREADS, tc_smem_bytes<CfgGroupedI8>(), st>>>(j->targs);
+        tc_grouped_kernel<CfgGroupedI8><<<grid, CfgGroupedI8::THREADS, tc_smem_bytes<CfgGroupedI8, false>(), st>>>(j->targs);
         prof.stop();
     } else {
         ProfScope prof("tc_grouped_3xbf16", st);
-        tc_grouped_kernel<CfgGroupedBf16><<<grid, CfgGroupedBf16::THREADS, tc_smem_bytes<CfgGroupedBf16>(), st>>>(j->targs);
+        tc_grouped_kernel<CfgGroupedBf16><<<grid, CfgGroupedBf16::THREADS, tc_smem_bytes<CfgGroupedBf16, false>(), st>>>(j->targs);
         prof.stop();
     }
     count_launch();

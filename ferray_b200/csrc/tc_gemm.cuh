@@ -202,10 +202,22 @@ __device__ __forceinline__ void batch_operands(const TcArgs& p, int bz, int& za,
     zb = static_cast<int>(ib);
 }
 
-template <class Cfg>
+// Whether a kernel's epilogue stores through shared memory (4 KB per epilogue
+// warp beside the operand stages).  The CRT epilogue writes bytes and the Ozaki
+// one doubles, row by row.
+template <class Cfg, int WARPS>
+constexpr bool epi_staged() {
+    return (Cfg::EPI == EPI_I32 || Cfg::EPI == EPI_I16 || Cfg::EPI == EPI_F32 || Cfg::EPI == EPI_QMM) &&
+           Cfg::STAGES * Cfg::STAGE_BYTES + WARPS * 4096 + 2048 <= 227 * 1024;
+}
+
+// EPI: with the staging memory of the epilogue's stores.
+template <class Cfg, bool EPI = true>
 struct TcSmem {
+    static constexpr bool STAGED = EPI && epi_staged<Cfg, 4>();
     alignas(1024) uint8_t a[Cfg::STAGES][Cfg::NA][Cfg::A_TILE];
     alignas(1024) uint8_t b[Cfg::STAGES][Cfg::NB][Cfg::B_TILE];
+    uint4 epi[STAGED ? 4 : 1][STAGED ? 256 : 1];  // per epilogue warp
     uint64_t full[Cfg::STAGES];
     uint64_t empty[Cfg::STAGES];
     uint64_t acc_full[4];
@@ -215,6 +227,148 @@ struct TcSmem {
     int abort;
 };
 
+// Stores a warp's 32 x 32 block of 4-byte outputs, lane i holding row row0 + i,
+// through its 4 KB of shared memory: a store instruction then writes 4 whole
+// 128-byte row pieces instead of 16 bytes in each of 32 rows (the accumulators
+// come out of TMEM one row per lane).  B200, before and after: i8 8192 x 8192 x 512
+// 117 -> 66 us, 3072^3 33.2 -> 26.4; f16 split 2048^3 99 -> 84; bf16 1024^3 17.1 ->
+// 11.0.  C is read, where it is, the same way.  Up to 32 rows a single warp of the
+// tile stores, and the detour's latency costs more than the pieces save (i8 16 x 1024
+// x 1024 6.7 -> 7.6 us, 32 x 8192 x 8192 20.0 -> 21.0): those rows go straight out.
+template <class Cfg>
+__device__ __forceinline__ void store_block32(const TcArgs& p, int bz, int row0, int gcol0, const uint32_t (&out)[32],
+                                              uint4* st) {
+    const int lane = threadIdx.x % 32;
+    const bool reads = Cfg::EPI == EPI_F32 ? p.beta != 0.f : p.accumulate != 0;
+    if (p.M <= 32 && !reads && gcol0 + 32 <= p.N) {
+        uint32_t* d = static_cast<uint32_t*>(p.C) + bz * p.strideC + (long long)(row0 + lane) * p.ldc + gcol0;
+        if (p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(d) & 15) == 0) {
+            if (row0 + lane < p.M) {
+#pragma unroll
+                for (int j = 0; j < 32; j += 4)
+                    *reinterpret_cast<uint4*>(d + j) = make_uint4(out[j], out[j + 1], out[j + 2], out[j + 3]);
+            }
+            return;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)  // 16-byte pieces, rotated so that neither side meets bank conflicts
+        st[lane * 8 + (j ^ (lane & 7))] = make_uint4(out[4 * j], out[4 * j + 1], out[4 * j + 2], out[4 * j + 3]);
+    __syncwarp();
+    // this lane's piece of rows r0, r0 + 4, ...: shared slot (q ^ row mod 8), so
+    // one of two offsets by turns
+    const int q = lane % 8, r0 = lane / 8, col = gcol0 + 4 * q;
+    const uint4* s0 = st + r0 * 8 + (q ^ r0);
+    const uint4* s1 = st + r0 * 8 + (q ^ (r0 + 4));
+    uint32_t* d = static_cast<uint32_t*>(p.C) + bz * p.strideC + (long long)(row0 + r0) * p.ldc + col;
+    const long long step = 4 * p.ldc;
+    auto update = [&](uint32_t w, uint32_t old) {
+        if constexpr (Cfg::EPI == EPI_F32)
+            return __float_as_uint(fmaf(p.beta, __uint_as_float(old), __uint_as_float(w)));
+        else if constexpr (Cfg::EPI == EPI_QMM)
+            return __float_as_uint(__fadd_rn(__uint_as_float(old), __uint_as_float(w)));
+        else
+            return w + old;
+    };
+    const bool vec = gcol0 + 32 <= p.N && p.ldc % 4 == 0 &&
+                     (reinterpret_cast<uintptr_t>(d) & 15) == 0;  // the same for the whole warp
+    const int rows = p.M - row0 - r0;  // row r0 + 4 i exists: 4 i < rows
+    if (vec && !reads) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const uint4 v = (i & 1 ? s1 : s0)[32 * i];
+            if (4 * i < rows) *reinterpret_cast<uint4*>(d) = v;
+            d += step;
+        }
+    } else if (vec) {
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {  // 16 rows at a time: all reads of C before the stores
+            uint4 o[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (16 * h + 4 * i < rows) o[i] = *reinterpret_cast<const uint4*>(d + i * step);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint4 v = (i & 1 ? s1 : s0)[128 * h + 32 * i];
+                if (16 * h + 4 * i < rows)
+                    *reinterpret_cast<uint4*>(d) =
+                        make_uint4(update(v.x, o[i].x), update(v.y, o[i].y), update(v.z, o[i].z), update(v.w, o[i].w));
+                d += step;
+            }
+        }
+    } else {
+#pragma unroll 1
+        for (int i = 0; i < 8 && 4 * i < rows; ++i) {
+            const uint4 v = (i & 1 ? s1 : s0)[32 * i];
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (col + j < p.N) d[j] = reads ? update(w[j], d[j]) : w[j];
+            d += step;
+        }
+    }
+    __syncwarp();  // the next block reuses the shared memory
+}
+
+// The FP16 split's operand scaling, undone: 2^-(sA + sB) as the (up to three)
+// normal factors that mul_pow2 applies, in its order, found once per kernel.
+struct EpiScale {
+    bool on;
+    float f[3];
+};
+template <class Cfg>
+__device__ __forceinline__ EpiScale epi_scale(const TcArgs& p) {
+    EpiScale s{false, {1.f, 1.f, 1.f}};
+    if constexpr (Cfg::EPI == EPI_F32) {
+        if (p.f16_amax) {
+            int e = -(f16_scale_exp(p.f16_amax[0]) + f16_scale_exp(p.f16_amax[1]));
+            s.on = e != 0;
+            e = max(-300, min(300, e));
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int step = e > 120 ? 120 : e < -120 ? -120 : 0;
+                s.f[i] = __int_as_float((127 + step) << 23);
+                e -= step;
+            }
+            s.f[2] = __int_as_float((127 + e) << 23);
+        }
+    }
+    return s;
+}
+
+// Outputs of a lane's row before C is read: 32 columns from gcol0.
+template <class Cfg>
+__device__ __forceinline__ void epilogue_values(const TcArgs& p, const EpiScale& sc, int grow, int gcol0,
+                                                const uint32_t (&v)[Cfg::NACC][32], uint32_t (&out)[32]) {
+    if constexpr (Cfg::EPI == EPI_I32) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) out[j] = v[0][j];
+    } else if constexpr (Cfg::EPI == EPI_I16) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) out[j] = (v[0][j] << 16) + (v[1][j] << 8) + v[2][j];
+    } else if constexpr (Cfg::EPI == EPI_QMM) {
+        const uint32_t rs = static_cast<uint32_t>(p.row_sum[min(grow, p.M - 1)]);
+        const uint32_t azp = static_cast<uint32_t>(p.a_zp), bzp = static_cast<uint32_t>(p.b_zp);
+        const uint32_t kab = static_cast<uint32_t>(p.K) * azp * bzp;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            const uint32_t cs = gcol0 + j < p.N ? static_cast<uint32_t>(p.col_sum[gcol0 + j]) : 0u;
+            const uint32_t corr = v[0][j] - azp * cs - bzp * rs + kab;
+            // Separate roundings, as gemm/mod.rs:566-571 computes them (no FMA).
+            out[j] = __float_as_uint(__fmul_rn(p.scale, static_cast<float>(static_cast<int32_t>(corr))));
+        }
+    } else {  // EPI_F32
+        if (sc.on) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+                out[j] = __float_as_uint(p.alpha * (__uint_as_float(v[0][j]) * sc.f[0] * sc.f[1] * sc.f[2]));
+        } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) out[j] = __float_as_uint(p.alpha * __uint_as_float(v[0][j]));
+        }
+    }
+}
+
 template <class Cfg>
 __device__ __forceinline__ void epilogue_store(const TcArgs& p, int bz, int grow, int gcol0,
                                                const uint32_t (&v)[Cfg::NACC][32], int oz_grp = 0) {
@@ -222,79 +376,7 @@ __device__ __forceinline__ void epilogue_store(const TcArgs& p, int bz, int grow
     if (grow >= p.M) return;
     const int ncols = min(32, p.N - gcol0);
     if (ncols <= 0) return;
-    if constexpr (Cfg::EPI == EPI_I32 || Cfg::EPI == EPI_I16) {
-        int32_t* crow = static_cast<int32_t*>(p.C) + bz * p.strideC + (long long)grow * p.ldc + gcol0;
-        uint32_t out[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            if constexpr (Cfg::EPI == EPI_I32) {
-                out[j] = v[0][j];
-            } else {
-                out[j] = (v[0][j] << 16) + (v[1][j] << 8) + v[2][j];
-            }
-        }
-        const bool vec = ncols == 32 && (reinterpret_cast<uintptr_t>(crow) & 15) == 0;
-        if (vec) {
-            if (p.accumulate) {
-                // all loads before the first store: they overlap instead of
-                // waiting behind stores that might alias them
-                uint4 o[8];
-#pragma unroll
-                for (int q = 0; q < 8; ++q) o[q] = *reinterpret_cast<const uint4*>(crow + 4 * q);
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    out[4 * q] += o[q].x; out[4 * q + 1] += o[q].y;
-                    out[4 * q + 2] += o[q].z; out[4 * q + 3] += o[q].w;
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < 32; j += 4)
-                *reinterpret_cast<uint4*>(crow + j) = make_uint4(out[j], out[j + 1], out[j + 2], out[j + 3]);
-        } else {
-            // fully unrolled with a predicate: a runtime trip count would
-            // index `out` dynamically and move it to local memory
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                if (j < ncols) {
-                    uint32_t w = out[j];
-                    if (p.accumulate) w += static_cast<uint32_t>(crow[j]);
-                    crow[j] = static_cast<int32_t>(w);
-                }
-            }
-        }
-    } else if constexpr (Cfg::EPI == EPI_QMM) {
-        float* crow = static_cast<float*>(p.C) + bz * p.strideC + (long long)grow * p.ldc + gcol0;
-        const uint32_t rs = static_cast<uint32_t>(p.row_sum[grow]);
-        const uint32_t azp = static_cast<uint32_t>(p.a_zp), bzp = static_cast<uint32_t>(p.b_zp);
-        const uint32_t kab = static_cast<uint32_t>(p.K) * azp * bzp;
-        // every load of the chunk is issued before the first store (stores
-        // to C could alias the sums, which would serialise load -> store)
-        uint32_t cs[32];
-        float old[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            cs[j] = j < ncols ? static_cast<uint32_t>(p.col_sum[gcol0 + j]) : 0u;
-            old[j] = (p.accumulate && j < ncols) ? crow[j] : 0.f;
-        }
-        float out[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            const uint32_t corr = v[0][j] - azp * cs[j] - bzp * rs + kab;
-            // Separate roundings, as gemm/mod.rs:566-571 computes them (no FMA).
-            float o = __fmul_rn(p.scale, static_cast<float>(static_cast<int32_t>(corr)));
-            if (p.accumulate) o = __fadd_rn(old[j], o);
-            out[j] = o;
-        }
-        if (ncols == 32 && (reinterpret_cast<uintptr_t>(crow) & 15) == 0) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 4)
-                *reinterpret_cast<float4*>(crow + j) = make_float4(out[j], out[j + 1], out[j + 2], out[j + 3]);
-        } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-                if (j < ncols) crow[j] = out[j];
-        }
-    } else if constexpr (Cfg::EPI == EPI_CRT) {
+    if constexpr (Cfg::EPI == EPI_CRT) {
         // exact int32 product of two residue planes -> its CRT residue byte
         const int m = p.crt_m[oz_grp], y = p.crt_y[oz_grp];
         uint8_t* crow = static_cast<uint8_t*>(p.C) + oz_grp * p.crt_plane + (long long)grow * p.ldc + gcol0;
@@ -424,6 +506,22 @@ __device__ __forceinline__ void epilogue_store(const TcArgs& p, int bz, int grow
                 }
             }
         }
+    }
+}
+
+// A warp's 32 x 32 block of the tile, lane i holding row row0 + i; st: the
+// warp's staging memory (unused by the row-wise epilogues).
+template <class Cfg, bool STAGED>
+__device__ __forceinline__ void epilogue_block(const TcArgs& p, const EpiScale& sc, int bz, int row0, int gcol0,
+                                               const uint32_t (&v)[Cfg::NACC][32], uint4* st, int oz_grp = 0) {
+    if (row0 >= p.M || gcol0 >= p.N) return;  // the same for the whole warp
+    const int grow = row0 + static_cast<int>(threadIdx.x % 32);
+    if constexpr (STAGED) {
+        uint32_t out[32];
+        epilogue_values<Cfg>(p, sc, grow, gcol0, v, out);
+        store_block32<Cfg>(p, bz, row0, gcol0, out, st);
+    } else {
+        epilogue_store<Cfg>(p, bz, grow, gcol0, v, oz_grp);
     }
 }
 
@@ -604,6 +702,8 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
     } else {
         // ------------------------------------------------ epilogue
         const int ew = warp & 3;  // TMEM lane quarter this warp may access
+        constexpr bool STAGED = TcSmem<Cfg>::STAGED;
+        const EpiScale sc = epi_scale<Cfg>(p);
         int it = 0;
         if constexpr (Cfg::CHUNKED) {
             // Tensor-core FP32 accumulation truncates at every MMA, so long K
@@ -615,6 +715,11 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
                 int zo, bz, tm, tn, kb0, kb1;
                 unit_coords(p, t, zo, bz, tm, tn, kb0, kb1);
                 const int kchunk = p.kchunk > 0 ? p.kchunk : kb1 - kb0;
+                constexpr int READS = Cfg::BN / 32 * Cfg::NACC;
+                uint32_t v[2][32];
+                auto read = [&](uint32_t (&d)[32], uint32_t row_addr, int i) {
+                    tmem_ld_32x32b_x32(row_addr + (Cfg::NACC - 1 - i % Cfg::NACC) * Cfg::BN + i / Cfg::NACC * 32, d);
+                };
                 float run[Cfg::BN];
 #pragma unroll
                 for (int j = 0; j < Cfg::BN; ++j) run[j] = 0.f;
@@ -629,31 +734,30 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
                     const uint32_t row_addr =
                         tmem + (static_cast<uint32_t>(ew * 32) << 16) + buf * Cfg::ACC_COLS;
 #pragma unroll
-                    for (int c = 0; c < Cfg::BN / 32; ++c) {
+                    for (int i = 0; i < READS; ++i) {
                         // accumulators are summed smallest first: the last
-                        // (correction products) before acc 0 (hi * hi)
+                        // (correction products) before acc 0 (hi * hi); the next
+                        // read is in flight behind these adds
+                        if (i == 0) read(v[0], row_addr, 0);
+                        tmem_wait_ld(v[i & 1]);
+                        if (i + 1 < READS) read(v[(i + 1) & 1], row_addr, i + 1);
 #pragma unroll
-                        for (int q = Cfg::NACC - 1; q >= 0; --q) {
-                            uint32_t v[32];
-                            tmem_ld_32x32b_x32(row_addr + q * Cfg::BN + c * 32, v);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int j = 0; j < 32; ++j)
-                                run[c * 32 + j] = __fadd_rn(run[c * 32 + j], __uint_as_float(v[j]));
-                        }
+                        for (int j = 0; j < 32; ++j)
+                            run[i / Cfg::NACC * 32 + j] =
+                                __fadd_rn(run[i / Cfg::NACC * 32 + j], __uint_as_float(v[i & 1][j]));
                     }
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&s.acc_empty[buf]);
                 }
                 if (!ok) break;
-                const int grow = tm * Cfg::BM + ew * 32 + lane;
+                const int row0 = tm * Cfg::BM + ew * 32;
 #pragma unroll
                 for (int c = 0; c < Cfg::BN / 32; ++c) {
-                    uint32_t v[Cfg::NACC][32];
+                    uint32_t o[Cfg::NACC][32];
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) v[0][j] = __float_as_uint(run[c * 32 + j]);
-                    epilogue_store<Cfg>(p, zo, grow, tn * Cfg::BN + c * 32, v);
+                    for (int j = 0; j < 32; ++j) o[0][j] = __float_as_uint(run[c * 32 + j]);
+                    epilogue_block<Cfg, STAGED>(p, sc, zo, row0, tn * Cfg::BN + c * 32, o, s.epi[STAGED ? ew : 0]);
                 }
             }
         } else {
@@ -670,15 +774,30 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
                 tc_fence_after();
                 int zo, bz, tm, tn, kb0, kb1;
                 unit_coords(p, t, zo, bz, tm, tn, kb0, kb1);
-                const int grow = tm * Cfg::BM + ew * 32 + lane;
+                const int row0 = tm * Cfg::BM + ew * 32;
                 const uint32_t row_addr = tmem + (static_cast<uint32_t>(ew * 32) << 16) + buf * Cfg::ACC_COLS;
+                if constexpr (Cfg::NACC == 1 && STAGED) {
+                    uint32_t v[2][1][32];  // the next block in flight behind the stores of this one
+                    tmem_ld_32x32b_x32(row_addr, v[0][0]);
 #pragma unroll 1
-                for (int c = 0; c < Cfg::BN / 32; ++c) {
-                    uint32_t v[Cfg::NACC][32];
+                    for (int c = 0; c < Cfg::BN / 32; c += 2) {
 #pragma unroll
-                    for (int a = 0; a < Cfg::NACC; ++a) tmem_ld_32x32b_x32(row_addr + a * Cfg::BN + c * 32, v[a]);
-                    tmem_wait_ld();
-                    epilogue_store<Cfg>(p, zo, grow, tn * Cfg::BN + c * 32, v, gi);
+                        for (int h = 0; h < 2; ++h) {
+                            tmem_wait_ld(v[h][0]);
+                            if (c + h + 1 < Cfg::BN / 32) tmem_ld_32x32b_x32(row_addr + (c + h + 1) * 32, v[h ^ 1][0]);
+                            epilogue_block<Cfg, STAGED>(p, sc, zo, row0, tn * Cfg::BN + (c + h) * 32, v[h],
+                                                        s.epi[STAGED ? ew : 0], gi);
+                        }
+                    }
+                } else {
+#pragma unroll 1
+                    for (int c = 0; c < Cfg::BN / 32; ++c) {
+                        uint32_t v[Cfg::NACC][32];
+#pragma unroll
+                        for (int a = 0; a < Cfg::NACC; ++a) tmem_ld_32x32b_x32(row_addr + a * Cfg::BN + c * 32, v[a]);
+                        tmem_wait_ld();
+                        epilogue_block<Cfg, STAGED>(p, sc, zo, row0, tn * Cfg::BN + c * 32, v, s.epi[STAGED ? ew : 0], gi);
+                    }
                 }
                 tc_fence_before();
                 __syncwarp();
@@ -696,9 +815,9 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
     }
 }
 
-template <class Cfg>
+template <class Cfg, bool EPI = true>
 constexpr size_t tc_smem_bytes() {
-    return sizeof(TcSmem<Cfg>) + 1024;
+    return sizeof(TcSmem<Cfg, EPI>) + 1024;
 }
 
 }  // namespace fg

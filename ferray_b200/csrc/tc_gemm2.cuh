@@ -17,7 +17,7 @@
 //   empty[s]     each CTA: the leader's commit, multicast to the pair,
 //                frees stage s in both;
 //   acc_full[b]  each CTA: leader's commit (multicast) -> both epilogues;
-//   acc_empty[b] leader only: 4 epilogue warps of each CTA arrive (the
+//   acc_empty[b] leader only: the epilogue warps of each CTA arrive (the
 //                peer's remotely) before accumulator b is reused
 //                (up to 4 accumulator buffers when they fit in TMEM).
 // Loads carry no cluster multicast: each CTA reads its own half from HBM.
@@ -56,14 +56,19 @@ struct Tc2Cfg {
     static constexpr int ACC_COLS = NACC * BN;                     // per CTA
     static constexpr int ACC_BUFS = (4 * ACC_COLS <= 512) ? 4 : (2 * ACC_COLS <= 512) ? 2 : 1;
     static constexpr int TMEM_COLS = 512;
-    static constexpr int THREADS = 192;
+    // Epilogue warps: four, or eight (two per TMEM lane quarter, half of the
+    // columns each) where the chunk sums of 256 columns would not fit a thread's
+    // registers.
+    static constexpr int EPI_WARPS = CHUNKED && BN == 256 ? 8 : 4;
+    static constexpr int EPI_COLS = BN * 4 / EPI_WARPS;  // columns per epilogue warp
+    static constexpr int THREADS = 64 + 32 * EPI_WARPS;
     static_assert(ACC_COLS <= 512, "accumulators exceed TMEM");
     static_assert(BN % 32 == 0 && BN <= 256, "UMMA N (pair)");
     static_assert(CTA_N % B_CHUNK_ELEMS == 0, "B half must be whole 128-byte chunks");
     static_assert(!COLSPLIT || (NACC == NB && NOPS == NB && !CHUNKED), "column split: one acc per B");
 };
 
-// Single-accumulator view of a config for epilogue_store (column-split
+// Single-accumulator view of a config for its epilogue (column-split
 // accumulators are stored one at a time).
 template <class Cfg>
 struct Tc2EpiView {
@@ -72,8 +77,10 @@ struct Tc2EpiView {
 
 template <class Cfg>
 struct Tc2Smem {
+    static constexpr bool STAGED = epi_staged<Cfg, Cfg::EPI_WARPS>();
     alignas(1024) uint8_t a[Cfg::STAGES][Cfg::NA][Cfg::A_TILE];
     alignas(1024) uint8_t b[Cfg::STAGES][Cfg::NB][Cfg::B_TILE];
+    uint4 epi[STAGED ? Cfg::EPI_WARPS : 1][STAGED ? 256 : 1];  // per epilogue warp
     uint64_t full[Cfg::STAGES];
     uint64_t empty[Cfg::STAGES];
     uint64_t acc_full[4];
@@ -120,7 +127,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg::THREADS, 1)
         }
         for (int i = 0; i < 4; ++i) {
             mbar_init(&s.acc_full[i], 1);
-            mbar_init(&s.acc_empty[i], 8);  // 4 epilogue warps x 2 CTAs
+            mbar_init(&s.acc_empty[i], 2 * Cfg::EPI_WARPS);  // both CTAs' epilogue warps
         }
         mbar_init(&s.drain, 1);
         s.abort = 0;
@@ -278,17 +285,35 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg::THREADS, 1)
     } else {
         // ------------------------------------------------ epilogue (both CTAs)
         const int ew = warp & 3;
+        const int ecol = (warp - 2) / 4 * Cfg::EPI_COLS;  // first column of this warp
+        constexpr bool STAGED = Tc2Smem<Cfg>::STAGED;
+        uint4* st = s.epi[STAGED ? warp - 2 : 0];
+        const EpiScale sc = epi_scale<Cfg>(p);
         int it = 0;
         bool ok = true;
         for (int t = pair; t < total && ok; t += npairs) {
             int zo, bz, tm, tn, kb0, kb1;
             unit_coords(p, t, zo, bz, tm, tn, kb0, kb1);
-            const int grow = tm * Cfg::BM + static_cast<int>(rank) * Cfg::CTA_M + ew * 32 + lane;
+            const int row0 = tm * Cfg::BM + static_cast<int>(rank) * Cfg::CTA_M + ew * 32;
             if constexpr (Cfg::CHUNKED) {
                 const int kchunk = p.kchunk > 0 ? p.kchunk : kb1 - kb0;
-                float run[Cfg::BN];
+                // 16-column reads with eight epilogue warps (168 registers a thread)
+                constexpr int W = Cfg::EPI_WARPS == 8 ? 16 : 32;
+                constexpr int READS = Cfg::EPI_COLS / W * Cfg::NACC;
+                // the next read in flight behind the adds of this one, where the registers allow it
+                constexpr int AHEAD = Cfg::EPI_WARPS == 8 ? 0 : 1;
+                uint32_t v[AHEAD + 1][W];
+                // read i: columns of group i / NACC, accumulators last (corrections) first
+                auto read = [&](uint32_t (&d)[W], uint32_t row_addr, int i) {
+                    const uint32_t a = row_addr + (Cfg::NACC - 1 - i % Cfg::NACC) * Cfg::BN + i / Cfg::NACC * W;
+                    if constexpr (W == 32)
+                        tmem_ld_32x32b_x32(a, d);
+                    else
+                        tmem_ld_32x32b_x16(a, d);
+                };
+                float run[Cfg::EPI_COLS];
 #pragma unroll
-                for (int j = 0; j < Cfg::BN; ++j) run[j] = 0.f;
+                for (int j = 0; j < Cfg::EPI_COLS; ++j) run[j] = 0.f;
                 for (int kc0 = kb0; kc0 < kb1; kc0 += kchunk, ++it) {
                     const int buf = it % Cfg::ACC_BUFS;
                     const uint32_t acc_par = static_cast<uint32_t>((it / Cfg::ACC_BUFS) & 1);
@@ -298,18 +323,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg::THREADS, 1)
                     }
                     tc_fence_after();
                     const uint32_t row_addr =
-                        tmem + (static_cast<uint32_t>(ew * 32) << 16) + buf * Cfg::ACC_COLS;
+                        tmem + (static_cast<uint32_t>(ew * 32) << 16) + buf * Cfg::ACC_COLS + ecol;
 #pragma unroll
-                    for (int c = 0; c < Cfg::BN / 32; ++c) {
+                    for (int i = 0; i < READS; ++i) {
+                        if (i == 0 || !AHEAD) read(v[0], row_addr, i);
+                        tmem_wait_ld(v[i & AHEAD]);
+                        if (AHEAD && i + 1 < READS) read(v[(i + 1) & AHEAD], row_addr, i + 1);
 #pragma unroll
-                        for (int q = Cfg::NACC - 1; q >= 0; --q) {
-                            uint32_t v[32];
-                            tmem_ld_32x32b_x32(row_addr + q * Cfg::BN + c * 32, v);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int j = 0; j < 32; ++j)
-                                run[c * 32 + j] = __fadd_rn(run[c * 32 + j], __uint_as_float(v[j]));
-                        }
+                        for (int j = 0; j < W; ++j)
+                            run[i / Cfg::NACC * W + j] =
+                                __fadd_rn(run[i / Cfg::NACC * W + j], __uint_as_float(v[i & AHEAD][j]));
                     }
                     tc_fence_before();
                     __syncwarp();
@@ -317,11 +340,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg::THREADS, 1)
                 }
                 if (!ok) break;
 #pragma unroll
-                for (int c = 0; c < Cfg::BN / 32; ++c) {
-                    uint32_t v[Cfg::NACC][32];
+                for (int c = 0; c < Cfg::EPI_COLS / 32; ++c) {
+                    uint32_t o[Cfg::NACC][32];
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) v[0][j] = __float_as_uint(run[c * 32 + j]);
-                    epilogue_store<Cfg>(p, zo, grow, tn * Cfg::BN + c * 32, v);
+                    for (int j = 0; j < 32; ++j) o[0][j] = __float_as_uint(run[c * 32 + j]);
+                    epilogue_block<Cfg, STAGED>(p, sc, zo, row0, tn * Cfg::BN + ecol + c * 32, o, st);
                 }
             } else {
                 for (int gi = 0; gi < max(p.oz_groups, 1); ++gi) {
@@ -343,7 +366,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg::THREADS, 1)
                             uint32_t v[1][32];
                             tmem_ld_32x32b_x32(row_addr + a * Cfg::BN + c * 32, v[0]);
                             tmem_wait_ld();
-                            epilogue_store<Tc2EpiView<Cfg>>(p, zo, grow, tn * Cfg::TILE_N + a * Cfg::BN + c * 32, v);
+                            epilogue_block<Tc2EpiView<Cfg>, STAGED>(p, sc, zo, row0, tn * Cfg::TILE_N + a * Cfg::BN + c * 32, v, st);
+                        }
+                    }
+                } else if constexpr (Cfg::NACC == 1 && STAGED) {
+                    uint32_t v[2][1][32];  // the next block in flight behind the stores of this one
+                    tmem_ld_32x32b_x32(row_addr, v[0][0]);
+#pragma unroll 1
+                    for (int c = 0; c < Cfg::BN / 32; c += 2) {
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            tmem_wait_ld(v[h][0]);
+                            if (c + h + 1 < Cfg::BN / 32) tmem_ld_32x32b_x32(row_addr + (c + h + 1) * 32, v[h ^ 1][0]);
+                            epilogue_block<Cfg, STAGED>(p, sc, zo, row0, tn * Cfg::BN + (c + h) * 32, v[h], st, gi);
                         }
                     }
                 } else {
@@ -353,7 +388,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg::THREADS, 1)
 #pragma unroll
                         for (int a = 0; a < Cfg::NACC; ++a) tmem_ld_32x32b_x32(row_addr + a * Cfg::BN + c * 32, v[a]);
                         tmem_wait_ld();
-                        epilogue_store<Cfg>(p, zo, grow, tn * Cfg::BN + c * 32, v, gi);
+                        epilogue_block<Cfg, STAGED>(p, sc, zo, row0, tn * Cfg::BN + c * 32, v, st, gi);
                     }
                 }
                 tc_fence_before();

@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-    TcSmem<Cfg>& s = *reinterpret_cast<TcSmem<Cfg>*>(base);
+    TcSmem<Cfg, false>& s = *reinterpret_cast<TcSmem<Cfg, false>*>(base);
     const int warp = threadIdx.x / 32;
     const int lane = threadIdx.x % 32;
     volatile int* abort = &s.abort;

@@ -74,7 +74,7 @@ static fg_status launch_group(fg_ctx* ctx, const TcMaps& maps, TcArgs& args, cud
     FG_CUDA(attr_err);
     args.status = ctx->d_status;
     args.timeout_ns = 4000000000ull;
-    const long long tiles = (long long)args.tiles_m * args.tiles_n;
+    const long long tiles = (long long)std::max(args.splits, 1) * args.tiles_m * args.tiles_n;
     const int units = static_cast<int>(std::min<long long>(tiles, max_units));
     ProfScope prof(pair ? "tc_gemm2_ozaki_i8" : "tc_gemm_ozaki_i8", st);
     if constexpr (pair)
@@ -201,8 +201,8 @@ static int inverse_mod(int a, int m) {  // a^-1 mod m (gcd(a, m) = 1)
 }
 
 // Constants of an n-moduli call with inner dimension K: P is the largest
-// integer precision (at most 59, so rint(x / m) in oz2_residue is off by at
-// most one) with K 2^(2P) < Mp / 4, i.e. every |C'| far from Mp / 2.
+// integer precision (at most 59: the residues take |a'| + 2^60 as 64-bit integers)
+// with K 2^(2P) < Mp / 4, i.e. every |C'| far from Mp / 2.
 static Oz2Consts oz2_consts(int n, long long K) {
     Oz2Consts c{};
     c.n = n;
@@ -212,20 +212,48 @@ static Oz2Consts oz2_consts(int n, long long K) {
     while ((1ll << logk) < K) ++logk;
     c.P = std::min(59, (Mp.bits() - 1 - logk - 2) / 2);
     for (int l = 0; l < n; ++l) {
-        const int m = kOz2Moduli[l];
-        BigU W = Mp;
-        W.divmod(static_cast<uint32_t>(m));  // exact: Mp / m_l
-        c.m[l] = m;
-        c.inv_m[l] = 1.0 / m;
+        const uint32_t m = static_cast<uint32_t>(kOz2Moduli[l]);
+        c.m[l] = static_cast<int>(m);
         c.magic[l] = static_cast<uint32_t>(((1ull << 32) + m - 1) / m);
-        c.c20[l] = static_cast<uint32_t>((1ull << 20) % m);
-        c.c40[l] = static_cast<uint32_t>((1ull << 40) % m);
-        for (int d = 0; d < 4; ++d) c.W[l][d] = static_cast<double>(W.bits_at(40 * d, 40));
+        uint32_t pw = 1;
+        for (int b = 0; b < 8; ++b) {
+            (b < 4 ? c.c_lo : c.c_hi)[l] |= pw << (8 * (b % 4));
+            pw = pw * 256 % m;
+        }
+        c.corr[l] = (m / 2 + m - static_cast<uint32_t>((1ull << 60) % m)) % m;
     }
-    for (int d = 0; d < 4; ++d) c.Mc[d] = static_cast<double>(Mp.bits_at(40 * d, 40));
-    c.M_d = Mp.to_double();
-    c.inv_M = 1.0 / c.M_d;
+    auto digit = [](const BigU& x, int d) { return static_cast<double>(x.bits_at(33 * d, 33)); };
+    for (int t = 0; t < (n + 1) / 2; ++t) {
+        const bool two = 2 * t + 1 < n;
+        BigU W = Mp;  // the divisions are exact
+        W.divmod(static_cast<uint32_t>(kOz2Moduli[2 * t]));
+        if (two) W.divmod(static_cast<uint32_t>(kOz2Moduli[2 * t + 1]));
+        c.pm[t][0] = two ? static_cast<uint32_t>(kOz2Moduli[2 * t + 1]) : 1;
+        c.pm[t][1] = two ? static_cast<uint32_t>(kOz2Moduli[2 * t]) : 0;
+        for (int d = 0; d < 5; ++d) c.pW[t][d] = digit(W, d);
+    }
+    for (int d = 0; d < 5; ++d) c.Mc[d] = digit(Mp, d);
+    if (n <= 18) {  // four digits: the top one takes what is left
+        for (int t = 0; t < (n + 1) / 2; ++t) c.pW[t][3] += c.pW[t][4] * 0x1p33;
+        c.Mc[3] += c.Mc[4] * 0x1p33;
+    }
+    c.inv_M = 1.0 / Mp.to_double();
     return c;
+}
+
+// oz2_reconstruct_kernel for c.n moduli.
+template <int N>
+static void launch_reconstruct(const Gemm& g, const uint8_t* res, long long pitch, const double* rsc, const double* csc,
+                               const Oz2Consts& c, cudaStream_t st) {
+    if constexpr (N <= 20) {
+        if (c.n != N) return launch_reconstruct<N + 1>(g, res, pitch, rsc, csc, c, st);
+        const long long per = g.dtype == FG_C64 ? 64 : 128;  // columns a block
+        const dim3 grid(static_cast<unsigned>((g.N + per - 1) / per),
+                        static_cast<unsigned>(std::min<long long>((g.M + 7) / 8, 65535)));
+        auto kernel = g.dtype == FG_C64 ? oz2_reconstruct_kernel<N, true> : oz2_reconstruct_kernel<N, false>;
+        kernel<<<grid, dim3(32, 8), 0, st>>>(res, g.M, g.N, pitch, rsc, csc, static_cast<double*>(g.C), g.ldc,
+                                             g.alpha_re, g.beta_re, c);
+    }
 }
 
 static int oz2_y(int n, int l) {  // ((Mp / m_l) mod m_l)^-1 mod m_l
@@ -247,7 +275,8 @@ static fg_status launch_ozaki2(fg_ctx* ctx, const Gemm& g, int n, cudaStream_t s
     const long long Kp = round_up(std::max<long long>(Kw, 1), 128), Np = round_up(Nw, 16);
     const Oz2Consts c = oz2_consts(n, Kw);
     const size_t a_bytes = static_cast<size_t>(M * n * Kp), b_bytes = static_cast<size_t>(n * Kp * Np);
-    const size_t r_bytes = static_cast<size_t>(n * M * Nw);
+    // residue planes with whole 16-byte pieces a row (777 x 1001 x 555 by bytes: 560 us)
+    const size_t r_bytes = static_cast<size_t>(n * M * Np);
     const size_t n_sc = static_cast<size_t>(g.N);
     const size_t meta = (M + n_sc) * sizeof(double) + n_sc * sizeof(unsigned long long) +
                         2 * g.K * sizeof(unsigned long long) + g.K * sizeof(int);
@@ -265,33 +294,46 @@ static fg_status launch_ozaki2(fg_ctx* ctx, const Gemm& g, int n, cudaStream_t s
     FG_TRY(scale_operands(g, cplx, rsc, csc, cmax, kmax_a, kmax_b, shift, st));
     const double* A = static_cast<const double*>(g.A);
     const double* B = static_cast<const double*>(g.B);
-    oz2_residue_a_kernel<<<grid_for(M * Kp / 8), 256, 0, st>>>(A, M, g.K, g.lda, cplx ? 1 : 0, shift, rsc, a_all, Kp, c);
-    oz2_residue_b_kernel<<<grid_for(Kp * Np / 8), 256, 0, st>>>(B, g.K, g.N, g.ldb, cplx ? 1 : 0, shift, csc, b_all, Kp, Np, c);
+    // rows of 256 entries a warp, 8 rows a block; B's threads keep their columns' scales
+    // over about four rows where that still fills the chip
+    auto rows = [&](long long x, long long blocks_x, long long per) {
+        const long long all = (x + 7) / 8, few = std::max<long long>(all / per, 16ll * ctx->sm_count / blocks_x + 1);
+        return static_cast<unsigned>(std::min({all, few, 65535ll}));
+    };
+    const bool va = !cplx && g.lda % 2 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0;
+    const bool vb = !cplx && g.ldb % 2 == 0 && (reinterpret_cast<uintptr_t>(B) & 15) == 0;
+    const unsigned ax = static_cast<unsigned>((Kp + 255) / 256), bx = static_cast<unsigned>((Np + 255) / 256);
+    (va ? oz2_residue_a_kernel<true> : oz2_residue_a_kernel<false>)<<<dim3(ax, rows(M, ax, 4)), dim3(32, 8), 0, st>>>(
+        A, M, g.K, g.lda, cplx ? 1 : 0, shift, rsc, a_all, Kp, c);
+    (vb ? oz2_residue_b_kernel<true> : oz2_residue_b_kernel<false>)<<<dim3(bx, rows(Kp, bx, 4)), dim3(32, 8), 0, st>>>(
+        B, g.K, g.N, g.ldb, cplx ? 1 : 0, shift, csc, b_all, Kp, Np, c);
     count_launch(2);
     FG_CUDA(cudaGetLastError());
 
-    const bool pair = tune_lookup(TUNE_I8, M, Nw, Kp).variant == 2;
-    // one launch for all moduli up to about 24 M outputs; beyond, one launch
-    // per modulus keeps the CTAs' K positions in step for L2 reuse
-    // (DGEMM 8192: 9.9 ms against 11.2 ms fused)
-    const bool fused = fused_groups() && M * Nw <= (24ll << 20);
-    const int launches = fused ? 1 : n;
-    for (int L = 0; L < launches; ++L) {
+    // 256 x 256 tiles on CTA pairs or 128 x 256: a wave of pairs is about 1/8 shorter
+    // for K beyond 1024 (1500 x 700 x 3000, 16 moduli: 45 against 52 us, 2048^3 95
+    // against 107, 4096^3 648 against 732) and no shorter up to there (1024^3 29.5
+    // against 28.7); rows of padding count against it (128 x 4096 x 4096 56 against 49).
+    const long long tn = (Nw + 255) / 256, sms = ctx->sm_count;
+    const long long wp = (n * ((M + 255) / 256) * tn + sms / 2 - 1) / (sms / 2);
+    const long long ws = (n * ((M + 127) / 128) * tn + sms - 1) / sms;
+    const bool pair = Kp > 1024 && 8 * wp <= 9 * ws;
+    {  // one launch for all moduli
         TcMaps maps;
         TcArgs args{};
-        const long long kw = fused ? n * Kp : Kp;
+        const long long kw = n * Kp;
         {
             uint64_t dims[2] = {static_cast<uint64_t>(kw), static_cast<uint64_t>(M)};
             uint64_t strides[1] = {static_cast<uint64_t>(n * Kp)};
             uint32_t box[2] = {128, 128};
-            FG_TRY(encode_map(&maps.a[0], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, a_all + (fused ? 0 : L * Kp), dims,
+            FG_TRY(encode_map(&maps.a[0], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, a_all, dims,
                               strides, box));
         }
         {
             uint64_t dims[2] = {static_cast<uint64_t>(Nw), static_cast<uint64_t>(kw)};
             uint64_t strides[1] = {static_cast<uint64_t>(Np)};
             uint32_t box[2] = {128, 128};
-            FG_TRY(encode_map(&maps.b[0], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, b_all + (fused ? 0 : L * Kp * Np), dims,
+            FG_TRY(encode_map(&maps.b[0], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, b_all, dims,
                               strides, box));
         }
         args.M = static_cast<int>(M);
@@ -303,16 +345,16 @@ static fg_status launch_ozaki2(fg_ctx* ctx, const Gemm& g, int n, cudaStream_t s
         args.batch = 1;
         args.bdims = 1;
         args.bshape[0] = 1;
-        args.C = res + (fused ? 0 : L * M * Nw);
-        args.ldc = Nw;
+        args.C = res;
+        args.ldc = Np;
         args.oz_crt = 1;
-        args.oz_groups = fused ? n : 1;
+        args.splits = n;
         args.oz_kc_blocks = static_cast<int>(Kp / CfgCrt::BK);
-        args.crt_plane = M * Nw;
-        for (int q = 0; q < (fused ? n : 1); ++q) {
-            const int l = fused ? q : L;
-            args.crt_m[q] = kOz2Moduli[l];
-            args.crt_y[q] = oz2_y(n, l);
+        args.crt_plane = M * Np;
+        for (int l = 0; l < n; ++l) {
+            args.crt_m[l] = kOz2Moduli[l];
+            args.crt_y[l] = oz2_y(n, l);
+            args.crt_magic[l] = static_cast<int>(c.magic[l]);
         }
         args.ops[0] = TcOp{0, 0, 0, 1, 1};
         if (pair)
@@ -322,9 +364,7 @@ static fg_status launch_ozaki2(fg_ctx* ctx, const Gemm& g, int n, cudaStream_t s
     }
     {
         ProfScope prof("oz2_reconstruct", st);
-        oz2_reconstruct_kernel<<<grid_for(M * Nw), 256, 0, st>>>(
-            res, M, Nw, M * Nw, rsc, csc, static_cast<double*>(g.C), g.ldc, cplx ? static_cast<int>(g.N) : 0,
-            g.alpha_re, g.beta_re, c);
+        launch_reconstruct<12>(g, res, Np, rsc, csc, c, st);
         prof.stop();
         count_launch();
     }

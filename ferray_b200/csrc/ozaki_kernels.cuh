@@ -35,6 +35,17 @@ __device__ __forceinline__ unsigned long long abs_bits(double x) {
     return static_cast<unsigned long long>(__double_as_longlong(x)) & 0x7FFFFFFFFFFFFFFFull;
 }
 
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }  // |e| <= 1000
+
+// x 2^sh, |sh| <= 2000, with one rounding: what is beyond 1000 is multiplied first,
+// which is exact unless the result is zero or infinite anyway.  No branch: ldexp in
+// a loop over a row kept its loads from being in flight together (4096^2: row
+// scales 48 -> 37 us, column maxima 53 -> 25).
+__device__ __forceinline__ double scale_pow2(double x, int sh) {
+    const int b = max(-1000, min(1000, sh));
+    return (x * pow2(sh - b)) * pow2(b);
+}
+
 // 2^e with frexp(max) = m * 2^e, m in [0.5, 1); zero rows get 1, non-finite
 // rows get NaN so their outputs come out NaN.
 __device__ __forceinline__ double scale_from_max_bits(unsigned long long bits) {
@@ -75,9 +86,10 @@ static __global__ void ozaki_row_scale_kernel(const double* __restrict__ A, long
     for (long long row = blockIdx.x; row < M; row += gridDim.x) {
         const double* r = A + row * (cplx ? 2 * lda : lda);
         unsigned long long mx = 0;
+#pragma unroll 8
         for (long long k = threadIdx.x; k < len; k += blockDim.x) {
             const int sh = shift ? shift[cplx ? (k >> 1) : k] : 0;
-            mx = max(mx, abs_bits(ldexp(r[k], sh)));
+            mx = max(mx, abs_bits(scale_pow2(r[k], sh)));
         }
         mx = block_max_u64(mx);
         if (threadIdx.x == 0) scale[row] = scale_from_max_bits(mx);
@@ -98,13 +110,14 @@ static __global__ void ozaki_col_max_kernel(const double* __restrict__ B, long l
     if (j >= N) return;
     const long long k0 = blockIdx.y * rows_per, k1 = min(K, k0 + rows_per);
     unsigned long long mx = 0;
+#pragma unroll 8
     for (long long k = k0; k < k1; ++k) {
         const int sh = shift ? -shift[k] : 0;
         if (cplx) {
             const double2 v = reinterpret_cast<const double2*>(B)[k * ldb + j];
-            mx = max(mx, max(abs_bits(ldexp(v.x, sh)), abs_bits(ldexp(v.y, sh))));
+            mx = max(mx, max(abs_bits(scale_pow2(v.x, sh)), abs_bits(scale_pow2(v.y, sh))));
         } else {
-            mx = max(mx, abs_bits(ldexp(B[k * ldb + j], sh)));
+            mx = max(mx, abs_bits(scale_pow2(B[k * ldb + j], sh)));
         }
     }
     atomicMax(colmax_bits + j, mx);
@@ -119,6 +132,7 @@ static __global__ void ozaki_a_colmax_kernel(const double* __restrict__ A, long 
     if (k >= K) return;
     const long long i0 = blockIdx.y * rows_per, i1 = min(M, i0 + rows_per);
     unsigned long long mx = 0;
+#pragma unroll 8
     for (long long i = i0; i < i1; ++i) {
         if (cplx) {
             const double2 v = reinterpret_cast<const double2*>(A)[i * lda + k];
@@ -138,6 +152,7 @@ static __global__ void ozaki_b_rowmax_kernel(const double* __restrict__ B, long 
     for (long long row = blockIdx.x; row < K; row += gridDim.x) {
         const double* r = B + row * (cplx ? 2 * ldb : ldb);
         unsigned long long mx = 0;
+#pragma unroll 8
         for (long long j = threadIdx.x; j < len; j += blockDim.x) mx = max(mx, abs_bits(r[j]));
         mx = block_max_u64(mx);
         if (threadIdx.x == 0) out[row] = mx;
@@ -272,198 +287,272 @@ __global__ void ozaki_slice_b_kernel(const double* __restrict__ B, long long K, 
 struct Oz2Consts {
     int n, P;
     int m[24];
-    double inv_m[24];
-    uint32_t magic[24];         // ceil(2^32 / m_l)
-    uint32_t c20[24], c40[24];  // 2^20 mod m_l, 2^40 mod m_l
-    double inv_M;               // 1 / Mp, for the CRT quotient
-    double W[24][4];  // Mp / m_l in base-2^40 digits (W[l][0] least significant)
-    double Mc[4];     // Mp in base-2^40 digits
-    double M_d;       // Mp rounded to double
+    uint32_t magic[24];             // ceil(2^32 / m_l)
+    uint32_t c_lo[24], c_hi[24];    // bytes 256^b mod m_l of the two words of an integer
+    uint32_t corr[24];              // (m_l / 2 - 2^60) mod m_l
+    double inv_M;                   // 1 / Mp, for the CRT quotient
+    uint32_t pm[10][2];             // moduli pair (2t, 2t + 1): m_(2t+1), m_2t (1, 0 for a single last)
+    double pW[10][5];               // Mp / (m_2t m_(2t+1)) in base-2^33 digits, least significant first
+    double Mc[5];                   // Mp in base-2^33 digits
 };
 
-// Symmetric residue of the integer-valued double x (|x| <= 2^61) modulo m:
-// q = rint(x / m) is off by at most one, r = x - q m is exact (fma), and at
-// most two corrections bring r into [-(m/2), m - 1 - (m/2)].
-__device__ __forceinline__ int8_t oz2_residue(double x, int m, double inv_m) {
-    const double q = rint(x * inv_m);
-    int r = static_cast<int>(fma(-q, static_cast<double>(m), x));
-    const int lo = -(m / 2), hi = lo + m - 1;
-    r += r < lo ? m : 0;
-    r += r < lo ? m : 0;
-    r -= r > hi ? m : 0;
-    r -= r > hi ? m : 0;
-    return static_cast<int8_t>(r);
+// 1 / s of a power of two (or NaN).
+__device__ __forceinline__ double recip_pow2(double s) {
+    const int hi = __double2hiint(s);
+    if (static_cast<unsigned>(hi - 0x00100000) < 0x7FD00000u) return __hiloint2double(0x7FE00000 - hi, 0);
+    return 1.0 / s;
 }
 
-// An integer-valued double |a| <= 2^60 as a sign and three 20-bit limbs
-// (integer arithmetic from here on: one conversion per element, not one per
-// modulus).
-struct Oz2Limbs {
-    uint32_t u0, u1, u2;
-    bool neg;
-};
-
-__device__ __forceinline__ Oz2Limbs oz2_limbs(double a) {
-    const long long v = static_cast<long long>(a);  // exact: a is an integer
-    const unsigned long long u = static_cast<unsigned long long>(v < 0 ? -v : v);
-    return Oz2Limbs{static_cast<uint32_t>(u & 0xFFFFFu), static_cast<uint32_t>((u >> 20) & 0xFFFFFu),
-                    static_cast<uint32_t>(u >> 40), v < 0};
+// rint(v) + 2^60 of |v| <= 2^59 (a non-finite entry counts as zero: its row's or
+// column's NaN scale marks the outputs).
+__device__ __forceinline__ uint2 oz2_biased(double v) {
+    const bool finite = (__double2hiint(v) & 0x7FF00000) != 0x7FF00000;
+    const unsigned long long u = static_cast<unsigned long long>(finite ? __double2ll_rn(v) : 0ll) + (1ull << 60);
+    return make_uint2(static_cast<uint32_t>(u), static_cast<uint32_t>(u >> 32));
 }
 
-// Symmetric residue of the limbs' integer modulo m: x = u2 (2^40 mod m) +
-// u1 (2^20 mod m) + u0 < 2^30, x mod m by a multiply-high with
-// ceil(2^32 / m) (quotient exact or one too large) and one correction, then
-// the sign and the symmetric range [-(m/2), m - 1 - (m/2)].
-__device__ __forceinline__ uint32_t oz2_residue_limbs(const Oz2Limbs& a, uint32_t m, uint32_t magic,
-                                                      uint32_t c20, uint32_t c40) {
-    const uint32_t x = a.u2 * c40 + a.u1 * c20 + a.u0;
-    int r = static_cast<int>(x - __umulhi(x, magic) * m);
-    r += r < 0 ? static_cast<int>(m) : 0;  // r in [0, m)
-    if (a.neg) r = r ? static_cast<int>(m) - r : 0;
-    const int hi = static_cast<int>(m) - 1 - static_cast<int>(m / 2);
-    r -= r > hi ? static_cast<int>(m) : 0;
-    return static_cast<uint32_t>(r) & 0xFFu;
-}
-
-// Eight consecutive residues of one plane packed into 8 bytes.
-__device__ __forceinline__ uint2 oz2_pack8(const Oz2Limbs (&x)[8], const Oz2Consts& c, int l) {
-    const uint32_t m = static_cast<uint32_t>(c.m[l]), magic = c.magic[l], c20 = c.c20[l], c40 = c.c40[l];
-    uint32_t w[2] = {0u, 0u};
+// Symmetric residues in [-(m/2), m - 1 - (m/2)] of eight such integers, packed.
+// The integer's bytes times 256^b mod m (two dp4a) give an x < 2^20 of the same
+// residue, x mod m is the high word of (x ceil(2^32 / m) mod 2^32) m, and m/2,
+// added before, is taken off all four bytes of a word at once.
+__device__ __forceinline__ uint2 oz2_pack8(const uint2 (&a)[8], const Oz2Consts& c, int l) {
+    const uint32_t m = static_cast<uint32_t>(c.m[l]), magic = c.magic[l], c_lo = c.c_lo[l], c_hi = c.c_hi[l];
+    const uint32_t corr = c.corr[l], h4 = (m / 2) * 0x01010101u;
+    uint32_t w[2];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) w[u / 4] |= oz2_residue_limbs(x[u], m, magic, c20, c40) << (8 * (u % 4));
+    for (int q = 0; q < 2; ++q) {
+        uint32_t r[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            r[u] = __umulhi(__dp4a(a[4 * q + u].x, c_lo, __dp4a(a[4 * q + u].y, c_hi, corr)) * magic, m);
+        const uint32_t p = __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
+        w[q] = ((p | 0x80808080u) - (h4 & 0x7F7F7F7Fu)) ^ ((p ^ ~h4) & 0x80808080u);
+    }
     return make_uint2(w[0], w[1]);
 }
 
 // A residue planes: A_all[i, l*Kp + k] = a'_ik mod m_l (complex A embedded
 // as [Ar | Ai], width 2K; columns past the width are zero).  A thread takes
-// eight consecutive k of one row and writes 8 bytes per plane.
-__global__ void oz2_residue_a_kernel(const double* __restrict__ A, long long M, long long K,
-                                     long long lda, int cplx, const int* __restrict__ shift,
-                                     const double* __restrict__ scale, int8_t* __restrict__ out,
-                                     long long Kp, const __grid_constant__ Oz2Consts c) {
+// eight consecutive k of one row and writes 8 bytes per plane; a block is 8 rows
+// of 256 k.  Instructions per entry and modulus bound it, about six (4096^2, 16
+// moduli: 127 us; 234 with three-limb residues and ldexp).
+// VEC: real A whose rows start on 16 bytes.
+template <bool VEC>
+__global__ void __launch_bounds__(256, 4) oz2_residue_a_kernel(
+    const double* __restrict__ A, long long M, long long K, long long lda, int cplx, const int* __restrict__ shift,
+    const double* __restrict__ scale, int8_t* __restrict__ out, long long Kp, const __grid_constant__ Oz2Consts c) {
     const long long W = cplx ? 2 * K : K;
-    const long long K8 = Kp / 8, total = M * K8;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-         e += (long long)gridDim.x * blockDim.x) {
-        const long long i = e / K8, k0 = (e - i * K8) * 8;
-        const double inv = 1.0 / scale[i];
-        Oz2Limbs a[8];
+    const long long k0 = (blockIdx.x * 32ll + threadIdx.x) * 8;
+    if (k0 >= Kp) return;
+    double f[8];  // of the shifts up to 1000; `more`: some go beyond
+    bool more = false;
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const long long k = k0 + u;
-            double x = 0.0;
-            if (k < W) {
-                if (cplx) {
-                    const long long kk = k < K ? k : k - K;
-                    x = ldexp(A[2 * (i * lda + kk) + (k < K ? 0 : 1)], shift[kk]);
-                } else {
-                    x = ldexp(A[i * lda + k], shift[k]);
-                }
+    for (int u = 0; u < 8; ++u) {
+        const long long k = k0 + u;
+        const int sh = k < W ? shift[k < K ? k : k - K] : 0, b = max(-1000, min(1000, sh));
+        f[u] = pow2(b);
+        more |= sh != b;
+    }
+    const double up = pow2(c.P);
+    for (long long i = blockIdx.y * 8ll + threadIdx.y; i < M; i += gridDim.y * 8ll) {
+        const double inv = recip_pow2(scale[i]);
+        double x[8];
+        if (VEC && k0 + 8 <= K) {
+#pragma unroll
+            for (int u = 0; u < 8; u += 2) {
+                const double2 v = *reinterpret_cast<const double2*>(A + i * lda + k0 + u);
+                x[u] = v.x;
+                x[u + 1] = v.y;
             }
-            double v = rint(ldexp(x * inv, c.P));
-            if (!isfinite(v)) v = 0.0;  // the row's NaN scale marks its outputs
-            a[u] = oz2_limbs(v);
+        } else {
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const long long k = k0 + u;
+                x[u] = k >= W ? 0.0 : cplx ? A[2 * (i * lda + (k < K ? k : k - K)) + (k < K ? 0 : 1)] : A[i * lda + k];
+            }
         }
+        if (more) {
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const long long k = k0 + u;
+                const int sh = k < W ? shift[k < K ? k : k - K] : 0;
+                x[u] *= pow2(sh - max(-1000, min(1000, sh)));
+            }
+        }
+        uint2 a[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) a[u] = oz2_biased((x[u] * f[u] * inv) * up);
         int8_t* o = out + i * (c.n * Kp) + k0;
         for (int l = 0; l < c.n; ++l) *reinterpret_cast<uint2*>(o + l * Kp) = oz2_pack8(a, c, l);
     }
 }
 
 // B residue planes: B_all[l*Kp + k, j] = b'_kj mod m_l (complex B embedded
-// as [[Br, Bi], [-Bi, Br]]).  A thread takes eight consecutive j of one row.
-__global__ void oz2_residue_b_kernel(const double* __restrict__ B, long long K, long long N,
-                                     long long ldb, int cplx, const int* __restrict__ shift,
-                                     const double* __restrict__ scale, int8_t* __restrict__ out,
-                                     long long Kp, long long Np, const __grid_constant__ Oz2Consts c) {
+// as [[Br, Bi], [-Bi, Br]]).  A thread takes eight consecutive j, whose scales it
+// keeps over its rows; bound as for A (122 us; 239 before).
+template <bool VEC>
+__global__ void __launch_bounds__(256, 4) oz2_residue_b_kernel(
+    const double* __restrict__ B, long long K, long long N, long long ldb, int cplx, const int* __restrict__ shift,
+    const double* __restrict__ scale, int8_t* __restrict__ out, long long Kp, long long Np,
+    const __grid_constant__ Oz2Consts c) {
     const long long H = cplx ? 2 * K : K, Wn = cplx ? 2 * N : N;
-    const long long N8 = Np / 8, total = Kp * N8;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-         e += (long long)gridDim.x * blockDim.x) {
-        const long long k = e / N8, j0 = (e - k * N8) * 8;
-        Oz2Limbs b[8];
+    const long long j0 = (blockIdx.x * 32ll + threadIdx.x) * 8;
+    if (j0 >= Np) return;
+    const double up = pow2(c.P);
+    double inv[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const long long j = j0 + u;
-            double x = 0.0, sc = 1.0;
-            if (k < H && j < Wn) {
-                if (cplx) {
-                    const bool top = k < K, left = j < N;
-                    const long long kk = top ? k : k - K, jj = left ? j : j - N;
-                    const double2 v = reinterpret_cast<const double2*>(B)[kk * ldb + jj];
-                    x = ldexp(top ? (left ? v.x : v.y) : (left ? -v.y : v.x), -shift[kk]);
-                    sc = scale[jj];
+    for (int u = 0; u < 8; ++u) {
+        const long long j = j0 + u;
+        inv[u] = j < Wn ? recip_pow2(scale[j < N ? j : j - N]) : 1.0;
+    }
+    for (long long k = blockIdx.y * 8ll + threadIdx.y; k < Kp; k += gridDim.y * 8ll) {
+        const bool top = k < K;
+        const long long kk = top ? k : k - K;
+        const int sh = k < H ? -shift[kk] : 0;
+        double x[8];
+        if (VEC && top && j0 + 8 <= N) {
+#pragma unroll
+            for (int u = 0; u < 8; u += 2) {
+                const double2 v = *reinterpret_cast<const double2*>(B + k * ldb + j0 + u);
+                x[u] = v.x;
+                x[u + 1] = v.y;
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const long long j = j0 + u;
+                const bool left = j < N;
+                if (k >= H || j >= Wn) {
+                    x[u] = 0.0;
+                } else if (cplx) {
+                    const double v = B[2 * (kk * ldb + (left ? j : j - N)) + (top == left ? 0 : 1)];
+                    x[u] = !top && left ? -v : v;
                 } else {
-                    x = ldexp(B[k * ldb + j], -shift[k]);
-                    sc = scale[j];
+                    x[u] = B[k * ldb + j];
                 }
             }
-            double v = rint(ldexp(x * (1.0 / sc), c.P));
-            if (!isfinite(v)) v = 0.0;
-            b[u] = oz2_limbs(v);
         }
-        for (int l = 0; l < c.n; ++l)
-            *reinterpret_cast<uint2*>(out + (l * Kp + k) * Np + j0) = oz2_pack8(b, c, l);
+        uint2 b[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) b[u] = oz2_biased((scale_pow2(x[u], sh) * inv[u]) * up);
+        int8_t* o = out + k * Np + j0;
+        for (int l = 0; l < c.n; ++l) *reinterpret_cast<uint2*>(o + l * Kp * Np) = oz2_pack8(b, c, l);
     }
 }
 
-// C from the residue bytes R[l][i, j] = (C'_ij mod m_l) y_l mod m_l:
-// S = sum_l R_l Mp/m_l is summed exactly in four base-2^40 digit sums
-// (each below 2^53), q = rint(S / Mp) (S / Mp < n, and |C'| < Mp / 4 keeps
-// it far from a tie), C' = S - q Mp digit by digit (exact), the digits are
-// balanced into [-2^39, 2^39) with exact int64 carries and C' is evaluated
-// from the top digit down (relative error about 2^-52).  Then
-// C = alpha 2^(e_i + f_j - 2P) C' (+ beta C).  Complex: embedded column
-// j < N is Re of column j, j >= N Im of column j - N (interleaved C).
-__device__ __forceinline__ double oz2_rebuild(double s0, double s1, double s2, double s3,
-                                              const Oz2Consts& c) {
-    const double est = ((s3 * 0x1p120 + s2 * 0x1p80) + s1 * 0x1p40) + s0;
-    const double q = rint(est * c.inv_M);
-    long long d0 = static_cast<long long>(fma(-q, c.Mc[0], s0));
-    long long d1 = static_cast<long long>(fma(-q, c.Mc[1], s1));
-    long long d2 = static_cast<long long>(fma(-q, c.Mc[2], s2));
-    long long d3 = static_cast<long long>(fma(-q, c.Mc[3], s3));
-    const long long half = 1ll << 39;
-    long long cy = (d0 + half) >> 40;
-    d0 -= cy << 40;
-    d1 += cy;
-    cy = (d1 + half) >> 40;
-    d1 -= cy << 40;
-    d2 += cy;
-    cy = (d2 + half) >> 40;
-    d2 -= cy << 40;
-    d3 += cy;
-    double x = static_cast<double>(d3);
-    x = fma(x, 0x1p40, static_cast<double>(d2));
-    x = fma(x, 0x1p40, static_cast<double>(d1));
-    return fma(x, 0x1p40, static_cast<double>(d0));
+// C from the residue bytes R[l][i, j] = (C'_ij mod m_l) y_l mod m_l, |C'| < Mp / 4:
+// C' = sum_l R_l Mp / m_l - q Mp.  Two moduli at a time, R_a Mp / m_a + R_b Mp / m_b
+// = (R_a m_b + R_b m_a) Mp / (m_a m_b) with a factor below 2^17, so the sum is exact
+// in base-2^33 digit sums (each below 2^53: 33 bits, and the factors of all pairs
+// add up to less than 2^20); q = rint(sum / Mp) (at most n, far from a tie),
+// the digits of C' follow exactly and are balanced into [-2^32, 2^32] with exact
+// carries; the two lowest digits, then all above them, are joined and rounded, so the
+// result is within about 2^-53 of C'.  Then C = alpha 2^(e_i + f_j - 2P) C' (+ beta C).
+// Complex: embedded column j < N is Re of column j, j >= N Im of column j - N
+// (interleaved C).  FP64 and instruction issue bound it about evenly (some 70
+// FP64 operations an output at 16 moduli); a thread has four columns, so that one
+// load brings four bytes (two columns: 165 us).  4096^2, 16 moduli: 128 us; 241 with
+// one output a thread, one modulus at a time, base 2^40 and integer carries.
+template <int ND>
+__device__ __forceinline__ double oz2_rebuild(double (&d)[ND], const Oz2Consts& c) {
+    constexpr double B = 0x1p33, MAGIC = 0x1.8p52;
+    double est = d[ND - 1];
+#pragma unroll
+    for (int k = ND - 2; k >= 0; --k) est = fma(est, B, d[k]);
+    const double q = fma(est, c.inv_M, MAGIC) - MAGIC;
+#pragma unroll
+    for (int k = 0; k < ND; ++k) d[k] = fma(-q, c.Mc[k], d[k]);
+#pragma unroll
+    for (int k = 0; k + 1 < ND; ++k) {
+        const double cy = fma(d[k], 0x1p-33, MAGIC) - MAGIC;
+        d[k] = fma(-cy, B, d[k]);
+        d[k + 1] += cy;
+    }
+    double hi = d[ND - 1];
+#pragma unroll
+    for (int k = ND - 2; k >= 2; --k) hi = fma(hi, B, d[k]);
+    return fma(hi, 0x1p66, fma(d[1], B, d[0]));
 }
 
-// One thread per output (measured faster than 4 or 8 outputs a thread:
-// the digit sums are FP64-bound and fewer registers keep more warps
-// resident).  A residue byte r becomes the double r by the exact
-// 2^52 + r - 2^52 bit trick.
-__global__ void oz2_reconstruct_kernel(const uint8_t* __restrict__ R, long long M, long long Nw,
-                                       long long plane, const double* __restrict__ rsc,
-                                       const double* __restrict__ csc, double* __restrict__ C,
-                                       long long ldc, int cplx_half, double alpha, double beta,
-                                       const __grid_constant__ Oz2Consts c) {
-    const long long total = M * Nw;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-         e += (long long)gridDim.x * blockDim.x) {
-        const long long i = e / Nw, j = e - i * Nw;
-        double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-        for (int l = 0; l < c.n; ++l) {
-            const double r = __hiloint2double(0x43300000, R[l * plane + e]) - 0x1p52;
-            s0 = fma(r, c.W[l][0], s0);
-            s1 = fma(r, c.W[l][1], s1);
-            s2 = fma(r, c.W[l][2], s2);
-            s3 = fma(r, c.W[l][3], s3);
+template <int N, bool CPLX>
+__global__ void __launch_bounds__(256, 3) oz2_reconstruct_kernel(
+    const uint8_t* __restrict__ R, long long M, long long cols, long long pitch, const double* __restrict__ rsc,
+    const double* __restrict__ csc, double* __restrict__ C, long long ldc, double alpha, double beta,
+    const __grid_constant__ Oz2Consts c) {
+    constexpr int PAIRS = (N + 1) / 2, ND = N <= 18 ? 4 : 5;
+    // complex: even lanes take the real parts of four columns, odd lanes the imaginary
+    // ones, and each stores two of the columns
+    const int part = CPLX ? threadIdx.x & 1 : 0;
+    const long long j0 = (CPLX ? blockIdx.x * 16ll + threadIdx.x / 2 : blockIdx.x * 32ll + threadIdx.x) * 4;
+    const bool live = j0 < cols;
+    const long long plane = M * pitch;
+    const bool aligned = !CPLX || cols % 4 == 0;  // of the imaginary columns' bytes
+    const bool vec = j0 + 4 <= cols && (reinterpret_cast<uintptr_t>(C) & 15) == 0 && (CPLX || ldc % 2 == 0);
+    for (long long i = blockIdx.y * 8ll + threadIdx.y; i < M; i += gridDim.y * 8ll) {
+        const uint8_t* r = R + i * pitch + part * cols + (live ? j0 : 0);
+        uint32_t w[N];
+        if (aligned || part == 0) {
+#pragma unroll
+            for (int l = 0; l < N; ++l) w[l] = *reinterpret_cast<const uint32_t*>(r + l * plane);
+        } else {
+#pragma unroll
+            for (int l = 0; l < N; ++l) {
+                w[l] = 0;
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (j0 + u < cols) w[l] |= static_cast<uint32_t>(r[l * plane + u]) << (8 * u);
+            }
         }
-        const double x = oz2_rebuild(s0, s1, s2, s3, c);
-        const long long jc = cplx_half > 0 ? (j < cplx_half ? j : j - cplx_half) : j;
-        const double o = (x * (ldexp(rsc[i], -2 * c.P) * alpha)) * csc[jc];
-        double* dst = cplx_half > 0 ? C + 2 * (i * ldc + jc) + (j < cplx_half ? 0 : 1) : C + i * ldc + j;
-        *dst = beta != 0.0 ? fma(beta, *dst, o) : o;
+        const double rs = ldexp(rsc[i], -2 * c.P) * alpha;
+        double o[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            double d[ND];
+#pragma unroll
+            for (int k = 0; k < ND; ++k) d[k] = 0.0;
+#pragma unroll
+            for (int t = 0; t < PAIRS; ++t) {
+                uint32_t f = ((w[2 * t] >> (8 * u)) & 0xFFu) * c.pm[t][0];
+                if (2 * t + 1 < N) f += ((w[2 * t + 1 < N ? 2 * t + 1 : 0] >> (8 * u)) & 0xFFu) * c.pm[t][1];
+                const double v = __hiloint2double(0x43300000, static_cast<int>(f)) - 0x1p52;
+#pragma unroll
+                for (int k = 0; k < ND; ++k) d[k] = fma(v, c.pW[t][k], d[k]);
+            }
+            o[u] = oz2_rebuild<ND>(d, c) * rs * csc[j0 + u < cols ? j0 + u : 0];
+        }
+        if (CPLX) {
+            const double a = __shfl_xor_sync(0xFFFFFFFFu, part ? o[0] : o[2], 1);
+            const double b = __shfl_xor_sync(0xFFFFFFFFu, part ? o[1] : o[3], 1);
+            const double re[2] = {part ? a : o[0], part ? b : o[1]}, im[2] = {part ? o[2] : a, part ? o[3] : b};
+            double* dst = C + 2 * (i * ldc + j0 + 2 * part);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                if (j0 + 2 * part + u >= cols) break;
+                double x = re[u], y = im[u];
+                if (beta != 0.0) {
+                    x = fma(beta, dst[2 * u], x);
+                    y = fma(beta, dst[2 * u + 1], y);
+                }
+                if (vec) {
+                    *reinterpret_cast<double2*>(dst + 2 * u) = make_double2(x, y);
+                } else {
+                    dst[2 * u] = x;
+                    dst[2 * u + 1] = y;
+                }
+            }
+        } else {
+            double* dst = C + i * ldc + j0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (j0 + u >= cols) break;
+                if (beta != 0.0) o[u] = fma(beta, dst[u], o[u]);
+                if (!vec) dst[u] = o[u];
+            }
+            if (vec) {
+                *reinterpret_cast<double2*>(dst) = make_double2(o[0], o[1]);
+                *reinterpret_cast<double2*>(dst + 2) = make_double2(o[2], o[3]);
+            }
+        }
     }
 }
 

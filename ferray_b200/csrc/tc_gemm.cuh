@@ -125,9 +125,13 @@ struct TcArgs {
     // EPI_CRT (Ozaki scheme II): group gi is the product of residue planes gi
     // (A K blocks [gi oz_kc_blocks, (gi + 1) oz_kc_blocks), B rows the same),
     // written as the byte ((acc mod m) y) mod m, m = crt_m[gi], y = crt_y[gi],
-    // into plane gi of C (planes crt_plane bytes apart, row pitch ldc).
+    // into plane gi of C (planes crt_plane bytes apart, row pitch ldc).  A work
+    // unit is one group of one tile, all tiles of a group before the next group
+    // (splits = the groups): the CTAs' K positions stay in step for L2 reuse, and
+    // few tiles still fill the chip (1024^3, 16 moduli: 130 us with a tile's groups
+    // in one CTA and a slower epilogue, 29 us; 4096^3 767 -> 650).
     int oz_crt;
-    int crt_m[24], crt_y[24];
+    int crt_m[24], crt_y[24], crt_magic[24];  // magic = ceil(2^32 / m)
     long long crt_plane;
     TcOp ops[TC_MAX_OPS];
     DevStatus* status;
@@ -186,6 +190,16 @@ __device__ __forceinline__ void group_range(const TcArgs& p, int gi, int kb0, in
         g0 = kb0;
         g1 = kb1;
         b_koff = 0;
+    }
+}
+
+// The groups of work unit t.
+__device__ __forceinline__ void group_span(const TcArgs& p, int t, int& ga, int& gb) {
+    ga = 0;
+    gb = max(p.oz_groups, 1);
+    if (p.oz_crt) {
+        ga = t / (p.batch * p.tiles_m * p.tiles_n);
+        gb = ga + 1;
     }
 }
 
@@ -378,21 +392,27 @@ __device__ __forceinline__ void epilogue_store(const TcArgs& p, int bz, int grow
     if (ncols <= 0) return;
     if constexpr (Cfg::EPI == EPI_CRT) {
         // exact int32 product of two residue planes -> its CRT residue byte
-        const int m = p.crt_m[oz_grp], y = p.crt_y[oz_grp];
+        // (two divisions a value by `%` took 8 us a 128 x 256 tile, more than its
+        // MMAs up to K = 4096)
+        const int m = p.crt_m[oz_grp], y = p.crt_y[oz_grp], magic = p.crt_magic[oz_grp], my = m * y;
         uint8_t* crow = static_cast<uint8_t*>(p.C) + oz_grp * p.crt_plane + (long long)grow * p.ldc + gcol0;
         uint32_t pk[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) pk[q] = 0;
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
-            int r = static_cast<int32_t>(v[0][j]) % m;
-            r += r < 0 ? m : 0;
-            r = (r * y) % m;
-            pk[j / 4] |= static_cast<uint32_t>(r) << (8 * (j % 4));
+            // floor(x magic / 2^32) = floor(x / m + d), 0 <= d sgn(x) < |x| / 2^32: for
+            // the accumulator off by one at most, r in (-m / 2, 3 m / 2); for
+            // 0 <= t = (r + m) y < 2^18 exact
+            const int x = static_cast<int32_t>(v[0][j]);
+            const int r = x - __mulhi(x, magic) * m;
+            const uint32_t t = static_cast<uint32_t>(r * y + my);
+            const uint32_t res = t - __umulhi(t, static_cast<uint32_t>(magic)) * static_cast<uint32_t>(m);
+            pk[j / 4] |= res << (8 * (j % 4));
         }
-        if (ncols == 32 && (reinterpret_cast<uintptr_t>(crow) & 15) == 0) {
+        if (p.ldc % 16 == 0) {  // whole pieces up to the pitch (planes are 16-byte aligned)
             *reinterpret_cast<uint4*>(crow) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-            *reinterpret_cast<uint4*>(crow + 16) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+            if (gcol0 + 16 < p.ldc) *reinterpret_cast<uint4*>(crow + 16) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
         } else {
 #pragma unroll
             for (int j = 0; j < 32; ++j)
@@ -576,12 +596,13 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
             // (register bitmasks; an indexed array would live in local memory)
             uint32_t issued_mask = 0, issued_par = 0;
             bool ok = true;
-            const int groups = max(p.oz_groups, 1);
             for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
                 int zo, bz, tm, tn, za, zb, kb0, kb1;
                 unit_coords(p, t, zo, bz, tm, tn, kb0, kb1);
                 batch_operands(p, bz, za, zb);
-                for (int gi = 0; gi < groups && ok; ++gi) {
+                int ga, gb;
+                group_span(p, t, ga, gb);
+                for (int gi = ga; gi < gb && ok; ++gi) {
                 int g0, g1, b_koff;
                 group_range(p, gi, kb0, kb1, g0, g1, b_koff);
                 for (int kb = g0; kb < g1; ++kb) {
@@ -635,11 +656,12 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
             uint32_t phase = 0;
             int it = 0;  // accumulator units (tile x K chunk) issued so far
             bool ok = true;
-            const int groups = max(p.oz_groups, 1);
             for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
                 int zo, bz, tm, tn, kb0, kb1;
                 unit_coords(p, t, zo, bz, tm, tn, kb0, kb1);
-                for (int gi = 0; gi < groups && ok; ++gi) {
+                int ga, gb;
+                group_span(p, t, ga, gb);
+                for (int gi = ga; gi < gb && ok; ++gi) {
                 int g0, g1, b_koff;
                 group_range(p, gi, kb0, kb1, g0, g1, b_koff);
                 const int kchunk = (Cfg::CHUNKED && p.kchunk > 0) ? p.kchunk : g1 - g0;
@@ -761,10 +783,11 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
                 }
             }
         } else {
-            const int groups = max(p.oz_groups, 1);
             bool ok = true;
             for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-                for (int gi = 0; gi < groups; ++gi, ++it) {
+                int ga, gb;
+                group_span(p, t, ga, gb);
+                for (int gi = ga; gi < gb; ++gi, ++it) {
                 const int buf = it % Cfg::ACC_BUFS;
                 const uint32_t acc_par = static_cast<uint32_t>((it / Cfg::ACC_BUFS) & 1);
                 if (!mbar_wait(&s.acc_full[buf], acc_par, p.timeout_ns, p.status, 0x21, abort)) {

@@ -155,14 +155,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg::THREADS, 1)
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
-            const int groups = max(p.oz_groups, 1);  // fused Ozaki slice groups per tile
             for (int t = pair; t < total && ok; t += npairs) {
                 int zo, bz, tm, tn, za, zb, kb0, kb1;
                 unit_coords(p, t, zo, bz, tm, tn, kb0, kb1);
                 batch_operands(p, bz, za, zb);
                 const int row0 = tm * Cfg::BM + static_cast<int>(rank) * Cfg::CTA_M;
                 const int col0 = tn * Cfg::TILE_N + static_cast<int>(rank) * Cfg::CTA_N;
-                for (int gi = 0; gi < groups && ok; ++gi) {
+                int ga, gb;
+                group_span(p, t, ga, gb);
+                for (int gi = ga; gi < gb && ok; ++gi) {
                 int g0, g1, b_koff;
                 group_range(p, gi, kb0, kb1, g0, g1, b_koff);
                 for (int kb = g0; kb < g1; ++kb) {
@@ -220,11 +221,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg::THREADS, 1)
             uint32_t phase = 0;
             int it = 0;
             bool ok = true;
-            const int groups = max(p.oz_groups, 1);
             for (int t = pair; t < total && ok; t += npairs) {
                 int zo, bz, tm, tn, kb0, kb1;
                 unit_coords(p, t, zo, bz, tm, tn, kb0, kb1);
-                for (int gi = 0; gi < groups && ok; ++gi) {
+                int ga, gb;
+                group_span(p, t, ga, gb);
+                for (int gi = ga; gi < gb && ok; ++gi) {
                 int g0, g1, b_koff;
                 group_range(p, gi, kb0, kb1, g0, g1, b_koff);
                 const int kchunk = (Cfg::CHUNKED && p.kchunk > 0) ? p.kchunk : g1 - g0;
@@ -347,7 +349,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg::THREADS, 1)
                     epilogue_block<Cfg, STAGED>(p, sc, zo, row0, tn * Cfg::BN + ecol + c * 32, o, st);
                 }
             } else {
-                for (int gi = 0; gi < max(p.oz_groups, 1); ++gi) {
+                int ga, gb;
+                group_span(p, t, ga, gb);
+                for (int gi = ga; gi < gb; ++gi) {
                 const int buf = it % Cfg::ACC_BUFS;
                 const uint32_t acc_par = static_cast<uint32_t>((it / Cfg::ACC_BUFS) & 1);
                 ++it;

@@ -6,10 +6,15 @@
 // FMAs per warp instruction, so the issue slots and registers that the DFMA
 // kernel spends on 8 x 8 outer products are freed.
 //
-// CTA: 256 threads, 128 x 128 output tile, K blocks of 16, a 3-stage
-// cp.async ring in shared memory (8-byte copies with zero fill past the
-// matrix edges, so any leading dimension and alignment works).  Warps form
-// a 2 (M) x 4 (N) grid of 64 x 32 warp tiles = 8 x 4 MMA tiles of 8 x 8.
+// CTA: 128 threads, 64 x 64 or 128 x 64 output tile, K blocks of 16, a 3-stage
+// cp.async ring in shared memory (16-byte copies where the rows allow them, else
+// 8-byte ones, with zero fill past the matrix edges, so any leading dimension and
+// alignment works).  Warps form a 2 x 2 grid of 32 x 32 or 64 x 32 warp tiles of
+// 8 x 8 MMAs.  The DMMA pipe bounds it; one CTA of 256 threads and 128 x 128 an SM
+// waited at its barrier (2048^3 670 us), two or three small ones fill each other's
+// waits (560 us, 30.7 TFLOP/s).  FOLD: accumulation runs of `seg` K blocks, each
+// added to the sum of the earlier ones, so that a CTA with all of K rounds like the
+// split-K form with one run a CTA.
 // Fragments (m8n8k4, f64): A row = lane / 4, col = lane % 4; B row =
 // lane % 4, col = lane / 4; C row = lane / 4, cols 2 (lane % 4) + {0, 1}.
 // Shared layouts: A [m][k] with a 4-double pad (the 8 rows x 4 k of an A
@@ -32,14 +37,16 @@ namespace fg {
 template <int WARPS_M_, int WARPS_N_, int MT_>
 struct DmmaTile {
     static constexpr int WARPS_M = WARPS_M_, WARPS_N = WARPS_N_, MT = MT_;
-    static constexpr int BM = WARPS_M * MT * 8, BN = WARPS_N * 32, BK = FG_DMMA_BK, STAGES = 3, THREADS = 256;
-    static_assert(WARPS_M * WARPS_N == 8, "256 threads");
+    static constexpr int BM = WARPS_M * MT * 8, BN = WARPS_N * 32, BK = FG_DMMA_BK, STAGES = 3;
+    static constexpr int THREADS = 32 * WARPS_M * WARPS_N;
+    static constexpr int MIN_CTAS = THREADS == 256 ? 1 : BM * BN <= 64 * 64 ? 3 : 2;
     static constexpr int APAD = 4, BPAD = 4;
     static constexpr int A_ELEMS = BM * (BK + APAD);
     static constexpr int B_ELEMS = BK * (BN + BPAD);
     static constexpr size_t SMEM = size_t(STAGES) * (A_ELEMS + B_ELEMS) * sizeof(double);
 };
-using DmmaCfg = DmmaTile<2, 4, 8>;        // 128 x 128, warps of 64 x 32
+using DmmaCfg = DmmaTile<2, 2, 8>;        // 128 x 64, four warps of 64 x 32
+using DmmaCfg64 = DmmaTile<2, 2, 4>;      // 64 x 64, four warps of 32 x 32
 using DmmaSkinnyCfg = DmmaTile<1, 8, 4>;  // 32 x 256 for few rows, warps of 32 x 32
 
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool valid) {
@@ -47,6 +54,10 @@ __device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool val
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(s), "l"(gmem),
                  "r"(valid ? 8 : 0)
                  : "memory");
+}
+__device__ __forceinline__ void cp_async16z(void* smem, const void* gmem, int bytes) {
+    const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -60,12 +71,12 @@ __device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
                  : "d"(a), "d"(b));
 }
 
-template <class Cfg>
-__global__ void __launch_bounds__(256, 1)
+template <class Cfg, bool VEC = false, bool FOLD = false>
+__global__ void __launch_bounds__(Cfg::THREADS, Cfg::MIN_CTAS)
     dmma_gemm_f64_kernel(int M, int N, int K, double alpha, const double* __restrict__ A,
                          long long lda, const double* __restrict__ B, long long ldb, double beta,
                          double* __restrict__ C, long long ldc, BatchMap bm, int nbatch,
-                         int ksplit) {
+                         int ksplit, int seg) {
     constexpr int MT = Cfg::MT;
     extern __shared__ __align__(16) double dsm[];
     double* As = dsm;                                  // [STAGES][BM][BK + APAD]
@@ -90,21 +101,26 @@ __global__ void __launch_bounds__(256, 1)
         const int k0 = kb * Cfg::BK;
         double* as = As + stage * Cfg::A_ELEMS;
         double* bs = Bs + stage * Cfg::B_ELEMS;
+        constexpr int W = VEC ? 2 : 1;  // elements a copy
+        auto copy = [&](double* dst, const double* base, long long off, int left) {
+            if constexpr (VEC)
+                cp_async16z(dst, left > 0 ? base + off : base, left > 1 ? 16 : left > 0 ? 8 : 0);
+            else
+                cp_async8(dst, left > 0 ? base + off : base, left > 0);
+        };
 #pragma unroll
-        for (int i = 0; i < Cfg::BM * Cfg::BK / 256; ++i) {
-            const int e = tid + 256 * i;
+        for (int i = 0; i < Cfg::BM * Cfg::BK / W / Cfg::THREADS; ++i) {
+            const int e = (tid + Cfg::THREADS * i) * W;
             const int r = e / Cfg::BK, c = e % Cfg::BK;  // A: BK k per row
             const int gr = m0 + r, gk = k0 + c;
-            const bool ok = gr < M && gk < K;
-            cp_async8(as + r * (Cfg::BK + Cfg::APAD) + c, ok ? A + (long long)gr * lda + gk : A, ok);
+            copy(as + r * (Cfg::BK + Cfg::APAD) + c, A, (long long)gr * lda + gk, gr < M ? K - gk : 0);
         }
 #pragma unroll
-        for (int i = 0; i < Cfg::BK * Cfg::BN / 256; ++i) {
-            const int e = tid + 256 * i;
+        for (int i = 0; i < Cfg::BK * Cfg::BN / W / Cfg::THREADS; ++i) {
+            const int e = (tid + Cfg::THREADS * i) * W;
             const int r = e / Cfg::BN, c = e % Cfg::BN;  // B: BN n per row
             const int gk = k0 + r, gn = n0 + c;
-            const bool ok = gk < K && gn < N;
-            cp_async8(bs + r * (Cfg::BN + Cfg::BPAD) + c, ok ? B + (long long)gk * ldb + gn : B, ok);
+            copy(bs + r * (Cfg::BN + Cfg::BPAD) + c, B, (long long)gk * ldb + gn, gk < K ? N - gn : 0);
         }
     };
 
@@ -113,6 +129,26 @@ __global__ void __launch_bounds__(256, 1)
     for (int i = 0; i < MT; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    double sum[FOLD ? MT : 1][4][2];
+    if constexpr (FOLD) {
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) sum[i][j][0] = sum[i][j][1] = 0.0;
+    }
+    auto fold = [&] {  // ends an accumulation run
+        if constexpr (FOLD) {
+#pragma unroll
+            for (int i = 0; i < MT; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        sum[i][j][u] += acc[i][j][u];
+                        acc[i][j][u] = 0.0;
+                    }
+        }
+    };
 
 #pragma unroll
     for (int s = 0; s < Cfg::STAGES - 1; ++s) {
@@ -121,6 +157,7 @@ __global__ void __launch_bounds__(256, 1)
     }
     const int fr = lane / 4, fc = lane % 4;
     for (int kb = 0; kb < kblocks; ++kb) {
+        if (FOLD && kb > 0 && kb % seg == 0) fold();
         cp_async_wait<Cfg::STAGES - 2>();
         __syncthreads();  // stage kb landed for everyone; stage kb-1 is free
         {
@@ -146,6 +183,7 @@ __global__ void __launch_bounds__(256, 1)
         }
     }
     cp_async_wait<0>();
+    fold();
 
 #pragma unroll
     for (int i = 0; i < MT; ++i) {
@@ -158,7 +196,7 @@ __global__ void __launch_bounds__(256, 1)
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 if (c + u < N) {
-                    double v = alpha * acc[i][j][u];
+                    double v = alpha * (FOLD ? sum[FOLD ? i : 0][j][u] : acc[i][j][u]);
                     if (beta != 0.0) v = fma(beta, p[u], v);
                     p[u] = v;
                 }

@@ -70,47 +70,122 @@ static fg_status launch_simt_real(const Gemm& g, BatchMap bm, int splits_want, c
     return FG_OK;
 }
 
-// Plain DGEMM on the FP64 tensor path (DMMA), same split-K scheme.
-template <class Cfg = DmmaCfg>
-static fg_status launch_dmma(fg_ctx* ctx, const Gemm& g, BatchMap bm, int splits_want, cudaStream_t st) {
-    (void)ctx;
+// Plain DGEMM on the FP64 tensor path (DMMA): accumulation runs of kps * 64 along K,
+// `runs` of them one after the other in a CTA and `parts` such ranges of K as CTAs of
+// their own, whose sums a second pass combines.
+template <class Cfg, bool VEC, bool FOLD>
+static fg_status launch_dmma_as(const Gemm& g, BatchMap bm, int runs, int kps, int parts, cudaStream_t st) {
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(dmma_gemm_f64_kernel<Cfg>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    auto kernel = dmma_gemm_f64_kernel<Cfg, VEC, FOLD>;
+    std::call_once(once, [kernel] {
+        attr_err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         static_cast<int>(Cfg::SMEM));
     });
     FG_CUDA(attr_err);
-    constexpr long long KUNIT = 64;
-    const long long kunits = (g.K + KUNIT - 1) / KUNIT;
-    int kps = static_cast<int>(kunits);
-    const int splits = plan_splits(splits_want, static_cast<int>(kunits), g.M * g.N * g.batch,
-                                   sizeof(double), &kps);
-    if ((long long)splits * g.batch > 65535) return set_error(FG_ERR_UNSUPPORTED, "batch above 65535");
-    dim3 grid((g.N + Cfg::BN - 1) / Cfg::BN, (g.M + Cfg::BM - 1) / Cfg::BM, g.batch * splits);
+    if ((long long)parts * g.batch > 65535) return set_error(FG_ERR_UNSUPPORTED, "batch above 65535");
+    const int seg = kps * 64 / Cfg::BK;
+    dim3 grid((g.N + Cfg::BN - 1) / Cfg::BN, (g.M + Cfg::BM - 1) / Cfg::BM, g.batch * parts);
     const double* A = static_cast<const double*>(g.A);
     const double* B = static_cast<const double*>(g.B);
-    if (splits <= 1) {
-        dmma_gemm_f64_kernel<Cfg><<<grid, Cfg::THREADS, Cfg::SMEM, st>>>(
+    if (parts <= 1) {
+        kernel<<<grid, Cfg::THREADS, Cfg::SMEM, st>>>(
             (int)g.M, (int)g.N, (int)g.K, g.alpha_re, A, g.lda, B, g.ldb, g.beta_re,
-            static_cast<double*>(g.C), g.ldc, bm, g.batch, (int)g.K);
+            static_cast<double*>(g.C), g.ldc, bm, g.batch, (int)g.K, seg);
         count_launch();
         FG_CUDA(cudaGetLastError());
         return FG_OK;
     }
     Scratch ws;
     const long long out_elems = g.M * g.N * g.batch;
-    FG_TRY(ws.alloc(static_cast<size_t>(splits * out_elems) * sizeof(double), st));
+    FG_TRY(ws.alloc(static_cast<size_t>(parts * out_elems) * sizeof(double), st));
     BatchMap wbm = bm;
     wbm.c_bstride = g.M * g.N;
-    dmma_gemm_f64_kernel<Cfg><<<grid, Cfg::THREADS, Cfg::SMEM, st>>>(
+    kernel<<<grid, Cfg::THREADS, Cfg::SMEM, st>>>(
         (int)g.M, (int)g.N, (int)g.K, 1.0, A, g.lda, B, g.ldb, 0.0, static_cast<double*>(ws.p), g.N, wbm,
-        g.batch, (int)(kps * KUNIT));
-    splitk_reduce<double>(static_cast<const double*>(ws.p), splits, g.M, g.N, g.batch, static_cast<double*>(g.C), g.ldc,
+        g.batch, runs * kps * 64, seg);
+    splitk_reduce<double>(static_cast<const double*>(ws.p), parts, g.M, g.N, g.batch, static_cast<double*>(g.C), g.ldc,
         g.c_stride, g.alpha_re, g.beta_re, 0, st);
     count_launch(2);
     FG_CUDA(cudaGetLastError());
     return FG_OK;
+}
+
+template <class Cfg>
+static fg_status launch_dmma_fold(const Gemm& g, BatchMap bm, int runs, int kps, int parts, cudaStream_t st) {
+    // 16-byte copies where every row of A and B starts on 16 bytes
+    bool vec = g.lda % 2 == 0 && g.ldb % 2 == 0 &&
+               ((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B)) & 15) == 0;
+    for (int d = 0; d < 4; ++d) vec = vec && bm.a_bstride[d] % 2 == 0 && bm.b_bstride[d] % 2 == 0;
+    if constexpr (Cfg::BM == 64) {
+        if (runs > 1)
+            return vec ? launch_dmma_as<Cfg, true, true>(g, bm, runs, kps, parts, st)
+                       : launch_dmma_as<Cfg, false, true>(g, bm, runs, kps, parts, st);
+    }
+    return vec ? launch_dmma_as<Cfg, true, false>(g, bm, 1, kps, parts, st)
+               : launch_dmma_as<Cfg, false, false>(g, bm, 1, kps, parts, st);
+}
+
+// Few rows: 32 x 256 tiles, every run a CTA of its own.
+static fg_status launch_dmma_skinny(const Gemm& g, BatchMap bm, int splits_want, cudaStream_t st) {
+    const long long kunits = (g.K + 63) / 64;
+    int kps = static_cast<int>(kunits);
+    const int splits = plan_splits(splits_want, static_cast<int>(kunits), g.M * g.N * g.batch, sizeof(double), &kps);
+    return launch_dmma_fold<DmmaSkinnyCfg>(g, bm, 1, kps, splits, st);
+}
+
+// Microseconds of a DMMA launch: a unit's FMAs at 64 a cycle of its SM, over the
+// share of that rate which the CTAs together on an SM reach (three of 64 x 64 0.87,
+// two 0.74, one 0.53; two of 128 x 64 0.85, one 0.53), in groups of as many as fit,
+// and the combine pass.  Fitted on a B200 to 12 shapes from 200^3 to 4096 x 4096 x
+// 1024 with 1 to 8 parts.
+static double dmma_us(int sms, const Gemm& g, bool wide, long long k_part, int parts) {
+    static const double share[2][3] = {{0.53, 0.74, 0.87}, {0.53, 0.85, 0.85}};
+    const int res = wide ? 2 : 3;
+    const long long bm = wide ? 128 : 64;
+    const long long units = (g.M + bm - 1) / bm * ((g.N + 63) / 64) * g.batch * parts, n = (units + sms - 1) / sms;
+    const double unit = static_cast<double>(bm * k_part) / 1930.0;
+    double us = n / res * (res * unit / share[wide][res - 1]);
+    if (n % res) us += n % res * unit / share[wide][n % res - 1];
+    if (parts > 1) us += 3.0 + (parts + 1.0) * g.M * g.N * g.batch / 1e6;
+    return us;
+}
+
+// Tile (128 x 64 or 64 x 64) and parts by that model; the accumulation runs are the
+// tuned split's, so results do not depend on the choice beyond the order in which
+// the runs' sums are added.  Against 128 x 128 tiles with every run a CTA of its own
+// (us): 768^3 74 -> 42, 1024^3 99 -> 90, 2048^3 670 -> 560, 4096 x 4096 x 1024 1194
+// -> 1088, 300 x 700 x 2000 92 -> 49, 1201 x 333 x 999 95 -> 55.
+// forced: a chosen variant of the table, 128 x 64 with `splits_want` parts.
+static fg_status launch_dmma(fg_ctx* ctx, const Gemm& g, BatchMap bm, int splits_want, bool forced, cudaStream_t st) {
+    const long long kunits = (g.K + 63) / 64;
+    int kps = static_cast<int>(kunits);
+    const int splits = plan_splits(splits_want, static_cast<int>(kunits), g.M * g.N * g.batch,
+                                   sizeof(double), &kps);
+    bool wide = true;
+    int parts = splits;
+    if (!forced) {
+        double best = 1e30;
+        for (int runs = splits; runs >= 1; --runs) {
+            const int p = (splits + runs - 1) / runs;
+            if (runs > 1 && p == (splits + runs - 2) / (runs - 1)) continue;  // fewer runs a part do as well
+            const long long k_part = std::min<long long>(g.K, (long long)runs * kps * 64);
+            for (int w = 0; w < 2; ++w) {
+                // 128 x 64 with two sums an output would spill; 64 rows a tile have to
+                // fit the grid
+                if (w ? runs > 1 : (g.M + 63) / 64 > 65535) continue;
+                const double us = dmma_us(ctx->sm_count, g, w != 0, k_part, p);
+                if (us < best) {
+                    best = us;
+                    wide = w != 0;
+                    parts = p;
+                }
+            }
+        }
+    }
+    const int runs = (splits + parts - 1) / parts;
+    return wide ? launch_dmma_fold<DmmaCfg>(g, bm, runs, kps, parts, st)
+                : launch_dmma_fold<DmmaCfg64>(g, bm, runs, kps, parts, st);
 }
 
 // ---- plain SGEMM on the cp.async FFMA kernel (ffma_sgemm.cuh)
@@ -381,8 +456,8 @@ fg_status launch_simt(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
                 case 1: return launch_simt_real<double, 4, 4>(g, bm, c.splits, st);
                 case 2: return launch_simt_real<double, 2, 8>(g, bm, c.splits, st);
                 case 3: return launch_simt_real<double, 8, 2>(g, bm, c.splits, st);
-                case 4: return launch_dmma(ctx, g, bm, c.splits, st);
-                case 5: return launch_dmma<DmmaSkinnyCfg>(ctx, g, bm, c.splits, st);
+                case 4: return launch_dmma(ctx, g, bm, c.splits, tune_forced(TUNE_F64), st);
+                case 5: return launch_dmma_skinny(g, bm, c.splits, st);
                 default: return launch_simt_real<double, 8, 8>(g, bm, c.splits, st);
             }
         }
@@ -438,7 +513,7 @@ fg_status launch_simt(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
                 r.ldb = 2 * g.N;
                 r.ldc = 2 * g.ldc;
                 const TuneChoice c = tune_lookup(TUNE_F64, r.M, r.N, r.K);
-                return launch_dmma(ctx, r, batch_map(r), c.variant == 4 ? c.splits : 1, st);
+                return launch_dmma(ctx, r, batch_map(r), c.variant == 4 ? c.splits : 1, false, st);
             }
             dim3 grid((g.N + 63) / 64, (g.M + 63) / 64, g.batch);
             simt_gemm_cplx<double, 8><<<grid, 256, 0, st>>>(

@@ -434,6 +434,12 @@ static fg_status launch_gemv(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
     return FG_OK;
 }
 
+// A plain DGEMM that leaves the table's variant for the small DMMA tiles.
+static bool small_dmma(const Gemm& g, const TuneChoice& c) {
+    if (c.variant == 5) return g.batch > 1 && g.N < 512;
+    return c.variant < 4 && g.K > (g.batch > 1 ? 8 : 16);
+}
+
 fg_status launch_simt(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
     if (g.batch == 1 && (g.N == 1 || g.M == 1) && (g.dtype == FG_F64 || g.dtype == FG_F32)) {
         ProfScope prof(g.dtype == FG_F64 ? "gemv_f64" : "gemv_f32", st);
@@ -445,18 +451,30 @@ fg_status launch_simt(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
     const char* fam = g.dtype <= FG_C32 ? names[g.dtype] : "simt";
     if (g.dtype == FG_F64 || g.dtype == FG_F32) {  // profile under the tuned kernel's name
         const TuneChoice c = tune_lookup(g.dtype == FG_F64 ? TUNE_F64 : TUNE_F32, g.M, g.N, g.K);
-        if (c.variant == 4) fam = g.dtype == FG_F64 ? "dmma_dgemm" : "ffma_sgemm";
-        if (c.variant == 5) fam = g.dtype == FG_F64 ? "dmma_dgemm_skinny" : "ffma_sgemm";
+        if (c.variant == 4 || (g.dtype == FG_F64 && small_dmma(g, c) && !tune_forced(TUNE_F64)))
+            fam = g.dtype == FG_F64 ? "dmma_dgemm" : "ffma_sgemm";
+        else if (c.variant == 5) fam = g.dtype == FG_F64 ? "dmma_dgemm_skinny" : "ffma_sgemm";
     }
     ProfScope prof(fam, st);
     switch (g.dtype) {
         case FG_F64: {
             const TuneChoice c = tune_lookup(TUNE_F64, g.M, g.N, g.K);
+            const bool forced = tune_forced(TUNE_F64);
+            // The register-staged tiles (0..3) only where they are chosen by hand: the
+            // small DMMA tiles do as well or better wherever the table (tuned with the
+            // 128 x 128 one) has them (100^3 15.6 -> 11.2 us, 400 x 300 x 100 17.9 ->
+            // 10.0, 500 x 120 x 900 20 -> 15, stacks of 128^3 x 100 51 -> 23, 250^3 x 16
+            // 59 -> 28, 33 x 65 x 129 x 500 101 -> 56).
+            // Outer products of up to 16 (one K block; in stacks 8) stay: 1000 x 1000 x 8
+            // 5.9 against 7.3 us, 128 x 128 x 8 x 100 8.4 against 8.9.  Stacks of few rows and less than two 32 x 256 tiles too
+            // (16^3 x 1000 18.6 -> 11.8, 10 x 300 x 300 x 8 18 -> 13; but 8 x 1000 x 1000
+            // x 4 24.6 against 28.6).
+            if (!forced && small_dmma(g, c)) return launch_dmma(ctx, g, bm, c.splits, false, st);
             switch (c.variant) {
                 case 1: return launch_simt_real<double, 4, 4>(g, bm, c.splits, st);
                 case 2: return launch_simt_real<double, 2, 8>(g, bm, c.splits, st);
                 case 3: return launch_simt_real<double, 8, 2>(g, bm, c.splits, st);
-                case 4: return launch_dmma(ctx, g, bm, c.splits, tune_forced(TUNE_F64), st);
+                case 4: return launch_dmma(ctx, g, bm, c.splits, forced, st);
                 case 5: return launch_dmma_skinny(g, bm, c.splits, st);
                 default: return launch_simt_real<double, 8, 8>(g, bm, c.splits, st);
             }

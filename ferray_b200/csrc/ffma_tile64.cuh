@@ -264,20 +264,24 @@ __device__ __forceinline__ void sgemm_tile64(const Tile64Args& p, int m0, int n0
     }
 }
 
-// Problem blockIdx.x of a stack, tile blockIdx.y: CTAs that run together work
-// on the same tile of different problems, so on the same one of the four
+// Problem blockIdx.x of a stack, tile blockIdx.z * gridDim.y + blockIdx.y (a grid's
+// y extent ends at 65535, a matrix may have more tiles): CTAs that run together
+// work on the same tile of different problems, so on the same one of the four
 // loops.
 template <bool VEC>
 static __global__ void __launch_bounds__(64, 6)
-    sgemm_tile64_kernel(Tile64Args p, BatchMap bm, int tiles_n, int chain) {
+    sgemm_tile64_kernel(Tile64Args p, BatchMap bm, int tiles_n, int tiles, int chain) {
     __shared__ Tile64Smem s;
     __shared__ Tile64Totals tot;
+    const int tile = static_cast<int>(blockIdx.z * gridDim.y + blockIdx.y);
+    if (tile >= tiles) return;
+    const int m0 = tile / tiles_n * 64, n0 = tile % tiles_n * 64;
     long long oa, ob;
     batch_offsets(bm, blockIdx.x, oa, ob);
     p.A += oa;
     p.B += ob;
     p.C += blockIdx.x * bm.c_bstride;
-    sgemm_tile64<VEC, true>(p, blockIdx.y / tiles_n * 64, blockIdx.y % tiles_n * 64, s, [] {}, [] {}, &tot, chain);
+    sgemm_tile64<VEC, true>(p, m0, n0, s, [] {}, [] {}, &tot, chain);
 }
 
 }  // namespace fg

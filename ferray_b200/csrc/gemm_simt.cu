@@ -382,11 +382,13 @@ static fg_status launch_tile64(const Gemm& g, const BatchMap& bm, TuneChoice tab
     const bool vec = g.lda % 4 == 0 && g.ldb % 4 == 0 &&
                      ((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B)) & 15) == 0 &&
                      (g.a_count == 1 || g.a_mstride % 4 == 0) && (g.b_count == 1 || g.b_mstride % 4 == 0);
-    const dim3 grid(static_cast<unsigned>(g.batch), static_cast<unsigned>(tm * tn));
+    const long long tiles = tm * tn, gy = std::min<long long>(tiles, 65535), gz = (tiles + gy - 1) / gy;
+    if (tiles > 0x7FFF0000ll) return set_error(FG_ERR_UNSUPPORTED, "stacked matrix above 2^31 tiles");
+    const dim3 grid(static_cast<unsigned>(g.batch), static_cast<unsigned>(gy), static_cast<unsigned>(gz));
     if (vec)
-        sgemm_tile64_kernel<true><<<grid, 64, 0, st>>>(a, bm, static_cast<int>(tn), chain);
+        sgemm_tile64_kernel<true><<<grid, 64, 0, st>>>(a, bm, static_cast<int>(tn), static_cast<int>(tiles), chain);
     else
-        sgemm_tile64_kernel<false><<<grid, 64, 0, st>>>(a, bm, static_cast<int>(tn), chain);
+        sgemm_tile64_kernel<false><<<grid, 64, 0, st>>>(a, bm, static_cast<int>(tn), static_cast<int>(tiles), chain);
     count_launch();
     FG_CUDA(cudaGetLastError());
     return FG_OK;

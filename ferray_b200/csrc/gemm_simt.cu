@@ -250,6 +250,7 @@ static FfmaChoice ffma_plan(int sms, long long M, long long N, long long K, long
             for (int t = 0; t < FFMA_TILES; ++t) {
                 if (only_tile >= 0 && t != only_tile) continue;
                 const FfmaTileInfo& f = kFfmaTiles[t];
+                if ((M + f.bm - 1) / f.bm > 65535) continue;  // the grid's y extent
                 const double work = 2.0 * f.bm * f.bn * kk / 1e3;  // us at 1 GFLOP/s
                 auto dur = [&](long long c) {
                     if (f.pairs) c = (c + 1) / 2 * 2;
@@ -269,10 +270,12 @@ static FfmaChoice ffma_plan(int sms, long long M, long long N, long long K, long
     return best;
 }
 
-// The packed transpose wants a K grid below 65536 blocks of 64, the kernel a
-// row grid below 65536 blocks of at least 16.
-constexpr long long kFfmaMaxK = 32LL * 65535;
-static bool ffma_ok(const Gemm& g) { return g.K <= kFfmaMaxK && g.M <= 16LL * 65535; }
+// The packed transpose wants a K grid below 65536 blocks of 64, the kernel a row
+// grid below 65536 blocks: of 128 rows, the planner leaves out the tiles that are
+// lower than M needs (2 M x 256 x 256: 4.9 ms, 7.4 register-staged; 1050000 x 160 x
+// 144: 1.25 against 2.10).
+static bool ffma_ok(long long M, long long K) { return K <= 32LL * 65535 && M <= 128LL * 65535; }
+static bool ffma_ok(const Gemm& g) { return ffma_ok(g.M, g.K); }
 
 // One launch: At packed, B in place, into C or (splits > 1) into partials.
 template <class Cfg>
@@ -548,7 +551,7 @@ fg_status launch_simt(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
             // GEMM (M x 2K) (2K x 2N) on it (same 8MNK flops, one FMA per
             // product); otherwise the 4M kernel.
             if (g.batch == 1 && g.alpha_im == 0.0 && g.beta_im == 0.0 && g.M > 0 && g.N > 0 && g.K > 0 &&
-                2 * g.K <= kFfmaMaxK && (reinterpret_cast<uintptr_t>(g.B) & 7) == 0) {
+                ffma_ok(g.M, 2 * g.K) && (reinterpret_cast<uintptr_t>(g.B) & 7) == 0) {
                 const TuneChoice c = tune_lookup(TUNE_F32, g.M, 2 * g.N, 2 * g.K);
                 if (c.variant == 4) {
                     Scratch bx;

@@ -237,6 +237,7 @@ struct FfmaChoice {
 // longest run of k that one accumulator may take (64-deep units): the size
 // table's split count also bounds the rounding error, which grows with the square
 // root of that run, so the model may split further than the table, never less.
+// us stays 1e300 where the grid's z extent (65535) leaves no such split.
 static FfmaChoice ffma_plan(int sms, long long M, long long N, long long K, long long batch, int fixed_splits,
                             int only_tile, int max_chain) {
     FfmaChoice best{std::max(only_tile, 0), std::max(fixed_splits, 1), 1e300};
@@ -244,7 +245,7 @@ static FfmaChoice ffma_plan(int sms, long long M, long long N, long long K, long
     for (int s = fixed_splits > 0 ? fixed_splits : 1;; ++s) {
         int kps = 0;
         const int ns = plan_splits(s, static_cast<int>(ku), M * N * batch, sizeof(float), &kps);
-        if (fixed_splits > 0 || (ns == s && (kps <= max_chain || s == TUNE_MAX_SPLITS))) {
+        if (fixed_splits > 0 || (ns == s && kps <= max_chain && ns * batch <= 65535)) {
             const double kk = static_cast<double>(std::min<long long>(K, 64LL * kps));
             const double combine = ns > 1 ? 3.0 + (2.0 * ns + 1) * M * N * 4 * batch / 5.0e6 : 0.0;
             for (int t = 0; t < FFMA_TILES; ++t) {
@@ -309,17 +310,28 @@ struct FfmaShifted<FfmaTile<BM, BN, TM, TN, MINB, BPAD, false>> {
 // launch_simt_real.  Results are bit-identical to simt_gemm_real<float, 8, 8, 8>
 // at equal split count.
 // `table`: the tuned choice for the shape (its split count fixed when forced).
-static fg_status launch_ffma(fg_ctx* ctx, const Gemm& g, TuneChoice table, int only_tile, cudaStream_t st) {
+// no_room(): what to do without memory for A's copy or the partial products.
+template <class NoRoom>
+static fg_status launch_ffma(fg_ctx* ctx, const Gemm& g, TuneChoice table, int only_tile, cudaStream_t st,
+                             NoRoom no_room) {
     const long long M = g.M, N = g.N, K = g.K;
     const long long Mp = (M + 3) / 4 * 4;
     const FfmaChoice c = ffma_plan(ctx->sm_count, M, N, K, g.batch, tune_forced(TUNE_F32) ? table.splits : 0, only_tile,
                                    chain_units(g, table.splits));
-    const long long kunits = (K + 63) / 64;
-    int kps = static_cast<int>(kunits);
-    int splits = plan_splits(c.splits, static_cast<int>(kunits), M * N * g.batch, sizeof(float), &kps);
-    if ((long long)splits * g.batch > 65535) splits = 1;  // the grid's z extent
+    const int kunits = static_cast<int>((K + 63) / 64);
+    int kps = kunits;
+    int splits = plan_splits(c.splits, kunits, M * N * g.batch, sizeof(float), &kps);
+    if ((long long)splits * g.batch > 65535) return set_error(FG_ERR_UNSUPPORTED, "batch above 65535");
     Scratch sa, ws;
-    FG_TRY(sa.alloc(static_cast<size_t>(g.a_count * K * Mp) * sizeof(float), st));
+    if (!sa.try_alloc(static_cast<size_t>(g.a_count * K * Mp) * sizeof(float), st)) return no_room();
+    if (splits > 1 && !ws.try_alloc(static_cast<size_t>(splits * M * N * g.batch) * sizeof(float), st)) {
+        // the table's own split count keeps the length of an accumulation run too
+        const int fewer = plan_splits(table.splits, kunits, M * N * g.batch, sizeof(float), &kps);
+        if (fewer >= splits) return no_room();
+        splits = fewer;
+        if (splits > 1 && !ws.try_alloc(static_cast<size_t>(splits * M * N * g.batch) * sizeof(float), st))
+            return no_room();
+    }
     float* At = static_cast<float*>(sa.p);
     transpose_pack_kernel<<<dim3(static_cast<unsigned>((Mp + 63) / 64), static_cast<unsigned>((K + 63) / 64),
                                  static_cast<unsigned>(g.a_count)),
@@ -330,8 +342,6 @@ static fg_status launch_ffma(fg_ctx* ctx, const Gemm& g, TuneChoice table, int o
     float* C = static_cast<float*>(g.C);
     long long ldc = g.ldc;
     float alpha = static_cast<float>(g.alpha_re), beta = static_cast<float>(g.beta_re);
-    // no room for the partial products: one split needs none
-    if (splits > 1 && ws.alloc(static_cast<size_t>(splits * M * N * g.batch) * sizeof(float), st) != FG_OK) splits = 1;
     if (splits > 1) {
         C = static_cast<float*>(ws.p);
         ldc = N;
@@ -363,6 +373,8 @@ static fg_status launch_ffma(fg_ctx* ctx, const Gemm& g, TuneChoice table, int o
     FG_CUDA(cudaGetLastError());
     return FG_OK;
 }
+
+static fg_status ffma_oom() { return set_error(FG_ERR_OOM, "no memory for the packed copy of A or the partial products"); }
 
 // Time of a stack by launch_tile64: a 16-deep K block takes 2.25 us with six CTAs
 // on an SM, 1 us alone, less where tiles have half the rows or columns (fit to
@@ -494,27 +506,27 @@ fg_status launch_simt(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
             // latency (191 x 37 x 44 x 32: 5.9 us, 8.3 with 64).
             if (!forced && g.batch > 1 && (g.M + 63) / 64 * ((g.N + 63) / 64) * g.batch > ctx->sm_count) {
                 const double packed = 4.0 + ffma_plan(ctx->sm_count, g.M, g.N, g.K, g.batch, 0, -1, chain_units(g, c.splits)).us;
-                if (!ffma_ok(g) || tile64_us(ctx->sm_count, g) < packed) return launch_tile64(g, bm, c, st);
-                return launch_ffma(ctx, g, c, -1, st);
+                auto tile64 = [&] { return launch_tile64(g, bm, c, st); };
+                if (!ffma_ok(g) || tile64_us(ctx->sm_count, g) < packed) return tile64();
+                return launch_ffma(ctx, g, c, -1, st, tile64);
             }
+            auto staged = [&] {
+                switch (c.variant) {
+                    case 1: return launch_simt_real<float, 4, 4>(g, bm, c.splits, st);
+                    case 2: case 5: return launch_simt_real<float, 2, 8>(g, bm, c.splits, st);
+                    case 3: return launch_simt_real<float, 8, 2>(g, bm, c.splits, st);
+                    default: return launch_simt_real<float, 8, 8>(g, bm, c.splits, st);
+                }
+            };
             // Deep problems that the table (tuned with the slower kernel this
             // family replaced) still gives a register-staged tile: 33 x 5675 x
             // 1040 47 -> 35 us, 220 x 130 x 3365 29 -> 25 us; below K = 1024 the
             // transpose launch costs more than it gives (279 x 195 x 802 17
             // against 21 us).
-            if (!forced && c.variant < 4 && g.K > 1024 && g.batch == 1 && ffma_ok(g)) return launch_ffma(ctx, g, c, -1, st);
-            switch (c.variant) {
-                case 1: return launch_simt_real<float, 4, 4>(g, bm, c.splits, st);
-                case 2: return launch_simt_real<float, 2, 8>(g, bm, c.splits, st);
-                case 3: return launch_simt_real<float, 8, 2>(g, bm, c.splits, st);
-                case 4:
-                    if (ffma_ok(g)) return launch_ffma(ctx, g, c, -1, st);
-                    return launch_simt_real<float, 8, 8>(g, bm, c.splits, st);
-                case 5:
-                    if (ffma_ok(g)) return launch_ffma(ctx, g, c, forced ? 4 : -1, st);
-                    return launch_simt_real<float, 2, 8>(g, bm, c.splits, st);
-                default: return launch_simt_real<float, 8, 8>(g, bm, c.splits, st);
-            }
+            if (!forced && c.variant < 4 && g.K > 1024 && g.batch == 1 && ffma_ok(g))
+                return launch_ffma(ctx, g, c, -1, st, staged);  // A's copy may not fit: those tiles need none
+            if (c.variant >= 4 && ffma_ok(g)) return launch_ffma(ctx, g, c, forced && c.variant == 5 ? 4 : -1, st, ffma_oom);
+            return staged();
         }
         case FG_C64: {
             // Real scalars and one output matrix: the real-embedded GEMM on
@@ -567,7 +579,7 @@ fg_status launch_simt(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
                     r.B = bx.p;
                     r.ldb = 2 * g.N;
                     r.ldc = 2 * g.ldc;
-                    return launch_ffma(ctx, r, c, -1, st);
+                    return launch_ffma(ctx, r, c, -1, st, ffma_oom);
                 }
             }
             dim3 grid((g.N + 63) / 64, (g.M + 63) / 64, g.batch);

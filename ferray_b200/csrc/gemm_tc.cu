@@ -183,19 +183,21 @@ static fg_status launch_any(fg_ctx* ctx, const TcMaps& maps, TcArgs& args, cudaS
 // Launches Cfg with up to `want` K splits (tuned).  With more than one
 // split the kernel writes dense partial products [split][batch][M][N] into a
 // workspace and splitk_reduce combines them into C (wrapping int32
-// sum + accumulate, or alpha * sum + beta * C).
+// sum + accumulate, or alpha * sum + beta * C).  unsplit_ok: without room for the
+// workspace one run over K serves (else that is an error, as it would also change
+// the rounding).
 template <class Cfg, typename T>
 static fg_status launch_splitk(fg_ctx* ctx, const TcMaps& maps, TcArgs& args, int want, T* C,
                                long long ldc, long long strideC, T alpha, T beta, int accumulate,
-                               cudaStream_t st) {
+                               cudaStream_t st, bool unsplit_ok = false) {
     const long long M = args.M, N = args.N, out_elems = M * N * args.batch;
     int kps = args.k_blocks;
     const int splits = plan_splits(want, args.k_blocks, out_elems, sizeof(T), &kps);
     if (splits <= 1) return launch_any<Cfg>(ctx, maps, args, st);
     Scratch ws;
-    // no room for the partial products: one split needs none
-    if (ws.alloc(static_cast<size_t>(splits * out_elems) * sizeof(T), st) != FG_OK)
-        return launch_any<Cfg>(ctx, maps, args, st);
+    const size_t bytes = static_cast<size_t>(splits * out_elems) * sizeof(T);
+    if (unsplit_ok && !ws.try_alloc(bytes, st)) return launch_any<Cfg>(ctx, maps, args, st);
+    if (!unsplit_ok) FG_TRY(ws.alloc(bytes, st));
     args.splits = splits;
     args.kb_per_split = kps;
     args.C = ws.p;
@@ -527,13 +529,10 @@ static fg_status launch_rows(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
         if (us < best) best = us, want = c;
     }
     int kps = k_blocks;
-    int splits = plan_splits(want, k_blocks, M * N, sizeof(float), &kps);
+    const int splits = plan_splits(want, k_blocks, M * N, sizeof(float), &kps);
     Scratch sp, ws;
     FG_TRY(sp.alloc(static_cast<size_t>(2 * pa * M) * sizeof(__nv_bfloat16), st));
-    if (splits > 1 && ws.alloc(static_cast<size_t>(splits * M * N) * sizeof(float), st) != FG_OK) {
-        splits = 1;  // no room for the partial products
-        kps = k_blocks;
-    }
+    if (splits > 1) FG_TRY(ws.alloc(static_cast<size_t>(splits * M * N) * sizeof(float), st));
     BfPlanes ap{};
     ap.p[0] = static_cast<__nv_bfloat16*>(sp.p);
     ap.p[1] = ap.p[0] + pa * M;
@@ -728,22 +727,24 @@ fg_status launch_split_bf16(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
     args.ops[0] = TcOp{1, 0, 0, sf, sf};  // lo * hi
     args.ops[1] = TcOp{0, 1, 0, sf, sf};  // hi * lo
     args.ops[2] = TcOp{0, 0, 0, sf, sf};  // hi * hi
-    const TuneChoice c = tune_lookup(TUNE_SPLIT_F32, M, N, K);  // tile variant and split-K
+    // Tile variant and split-K.  Complex products may run unsplit without room for
+    // the partial ones: their K runs have no tuned length to keep.
+    const TuneChoice c = tune_lookup(TUNE_SPLIT_F32, M, N, K);
     float* C = static_cast<float*>(g.C);
     const float alpha = args.alpha, beta = args.beta;
     if (c.variant == 2) {
         args.tiles_m = static_cast<int>((M + CfgBf16x3Pair::BM - 1) / CfgBf16x3Pair::BM);
         args.tiles_n = static_cast<int>((N + CfgBf16x3Pair::BN - 1) / CfgBf16x3Pair::BN);
         return launch_splitk<CfgBf16x3Pair, float>(ctx, maps, args, c.splits, C, ldc, c_ms,
-                                                   alpha, beta, 0, st);
+                                                   alpha, beta, 0, st, cplx);
     }
     if (c.variant == 1) {
         args.tiles_n = static_cast<int>((N + CfgBf16x3n64::BN - 1) / CfgBf16x3n64::BN);
         return launch_splitk<CfgBf16x3n64, float>(ctx, maps, args, c.splits, C, ldc, c_ms,
-                                                  alpha, beta, 0, st);
+                                                  alpha, beta, 0, st, cplx);
     }
     return launch_splitk<CfgBf16x3, float>(ctx, maps, args, c.splits, C, ldc, c_ms, alpha,
-                                           beta, 0, st);
+                                           beta, 0, st, cplx);
 }
 
 }  // namespace fgrt

@@ -86,16 +86,18 @@ struct Scratch {
     Scratch() = default;
     Scratch(const Scratch&) = delete;
     Scratch& operator=(const Scratch&) = delete;
-    fg_status alloc(size_t bytes, cudaStream_t stream) {
+    // False (and no error recorded) when there is no room: for callers that have
+    // another way to run.
+    bool try_alloc(size_t bytes, cudaStream_t stream) {
         st = stream;
-        if (bytes == 0) bytes = 16;
-        cudaError_t e = cudaMallocAsync(&p, bytes, stream);
-        if (e != cudaSuccess) {
-            p = nullptr;
-            cudaGetLastError();
-            return set_error(FG_ERR_OOM, "scratch allocation of " + std::to_string(bytes) + " bytes failed");
-        }
-        return FG_OK;
+        if (cudaMallocAsync(&p, bytes ? bytes : 16, stream) == cudaSuccess) return true;
+        p = nullptr;
+        cudaGetLastError();
+        return false;
+    }
+    fg_status alloc(size_t bytes, cudaStream_t stream) {
+        if (try_alloc(bytes, stream)) return FG_OK;
+        return set_error(FG_ERR_OOM, "scratch allocation of " + std::to_string(bytes) + " bytes failed");
     }
     ~Scratch() {
         if (p) cudaFreeAsync(p, st);

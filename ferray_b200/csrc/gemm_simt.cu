@@ -306,6 +306,34 @@ struct FfmaShifted<FfmaTile<BM, BN, TM, TN, MINB, BPAD, false>> {
     using type = FfmaTile<BM, BN, TM, TN, MINB, BPAD, true>;
 };
 
+// Every row of every one of these f32 matrices starts on 16 bytes.
+static bool rows16(const void* X, long long ld, long long count, long long mstride) {
+    return (reinterpret_cast<uintptr_t>(X) & 15) == 0 && ld % 4 == 0 && (count == 1 || mstride % 4 == 0);
+}
+
+// Deep problems that the table (tuned with the slower kernel this family replaced)
+// still gives a register-staged tile: does the packed kernel pay for its transpose of
+// A?  From 630 shapes of 33 to 30000 rows, 2 to 1000 columns and K from 1100 to 12000
+// (us, register-staged / packed):
+//  * not for up to K = 1024 (279 x 195 x 802 17 / 21);
+//  * with enough outputs to fill the chip, unless they are a few columns, where the
+//    copy of A is most of the work: 33 x 7000 x 1100 41 / 26, 3000 x 64 x 2000 37 /
+//    28, but 7000 x 9 x 3000 81 / 101, 1000 x 64 x 2000 21 / 23;
+//  * with few outputs where K is long and B comes in whole granules: 300 x 100 x
+//    6000 39 / 33, 64 x 20 x 12000 47 / 37, but 300 x 33 x 6000 28 / 31;
+//  * few rows of a wide B: 17 x 1000 x 3000 1.18 x;
+//  * where the table's 64 x 64 tiles times its splits just pass one wave: 220 x 130
+//    x 3365 29 / 25 (220 x 65 x 3365 22 / 25).
+static bool packed_pays(int sms, const Gemm& g, TuneChoice table) {
+    if (g.K <= 1024) return false;
+    if (g.N > 32 && g.M * g.N >= 90000) return true;
+    if (g.K >= 6000 && g.M <= 1000 && rows16(g.B, g.ldb, 1, 0)) return true;
+    if (table.variant == 2 && g.N >= 1000) return true;
+    int kps = 0;
+    const int splits = plan_splits(table.splits, static_cast<int>((g.K + 63) / 64), g.M * g.N, sizeof(float), &kps);
+    return table.variant == 1 && g.K > 3000 && g.N >= 100 && (g.M + 63) / 64 * ((g.N + 63) / 64) * splits > sms;
+}
+
 // A transposed into packed scratch, B in place, same split-K scheme as
 // launch_simt_real.  Results are bit-identical to simt_gemm_real<float, 8, 8, 8>
 // at equal split count.
@@ -350,8 +378,7 @@ static fg_status launch_ffma(fg_ctx* ctx, const Gemm& g, TuneChoice table, int o
         beta = 0.f;
     }
     const int ksplit = splits > 1 ? kps * 64 : static_cast<int>(K);
-    const bool aligned = (reinterpret_cast<uintptr_t>(g.B) & 15) == 0 && g.ldb % 4 == 0 &&
-                         (g.b_count == 1 || g.b_mstride % 4 == 0);
+    const bool aligned = rows16(g.B, g.ldb, g.b_count, g.b_mstride);
     auto run = [&](auto tile) {
         using T = decltype(tile);
         if (aligned) return launch_ffma_tile<T>(g, At, Mp, bm, splits, ksplit, alpha, beta, C, ldc, st);
@@ -394,9 +421,7 @@ static fg_status launch_tile64(const Gemm& g, const BatchMap& bm, TuneChoice tab
     const Tile64Args a{(int)g.M, (int)g.N, (int)g.K, static_cast<const float*>(g.A), static_cast<const float*>(g.B),
                        static_cast<float*>(g.C), g.lda, g.ldb, g.ldc, (float)g.alpha_re, (float)g.beta_re};
     const int chain = 4 * chain_units(g, table.splits);  // 16-deep K blocks
-    const bool vec = g.lda % 4 == 0 && g.ldb % 4 == 0 &&
-                     ((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B)) & 15) == 0 &&
-                     (g.a_count == 1 || g.a_mstride % 4 == 0) && (g.b_count == 1 || g.b_mstride % 4 == 0);
+    const bool vec = rows16(g.A, g.lda, g.a_count, g.a_mstride) && rows16(g.B, g.ldb, g.b_count, g.b_mstride);
     const long long tiles = tm * tn, gy = std::min<long long>(tiles, 65535), gz = (tiles + gy - 1) / gy;
     if (tiles > 0x7FFF0000ll) return set_error(FG_ERR_UNSUPPORTED, "stacked matrix above 2^31 tiles");
     const dim3 grid(static_cast<unsigned>(g.batch), static_cast<unsigned>(gy), static_cast<unsigned>(gz));
@@ -518,12 +543,7 @@ fg_status launch_simt(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
                     default: return launch_simt_real<float, 8, 8>(g, bm, c.splits, st);
                 }
             };
-            // Deep problems that the table (tuned with the slower kernel this
-            // family replaced) still gives a register-staged tile: 33 x 5675 x
-            // 1040 47 -> 35 us, 220 x 130 x 3365 29 -> 25 us; below K = 1024 the
-            // transpose launch costs more than it gives (279 x 195 x 802 17
-            // against 21 us).
-            if (!forced && c.variant < 4 && g.K > 1024 && g.batch == 1 && ffma_ok(g))
+            if (!forced && c.variant < 4 && g.batch == 1 && ffma_ok(g) && packed_pays(ctx->sm_count, g, c))
                 return launch_ffma(ctx, g, c, -1, st, staged);  // A's copy may not fit: those tiles need none
             if (c.variant >= 4 && ffma_ok(g)) return launch_ffma(ctx, g, c, forced && c.variant == 5 ? 4 : -1, st, ffma_oom);
             return staged();

@@ -619,10 +619,16 @@ fg_status launch_split_bf16(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
     const bool f16 = g.mode == FG_MODE_SPLIT_F16;  // two FP16 slices of scaled operands
     const int ns = (!f16 && g.slices == 3) ? 3 : 2;  // slices per operand
     // Up to 64 rows B is read once, so cutting it in a pass of its own triples the
-    // bytes: a call with 32 x 8192 x 8192 takes 64 us by the rows kernel against
-    // 156, 64 x 64 x 64 12.3 against 14.5 (36 shapes of 1-64 rows: 1.14-2.7x).
-    if (!cplx && !f16 && ns == 2 && g.batch == 1 && g.M <= 64 && !tune_forced(TUNE_SPLIT_F32)) {
-        const bool tma = tma_ok(g.B, g.ldb * 4, 1, 0);
+    // bytes: the kernels of a call with 32 x 8192 x 8192 take 64 us by the rows kernel
+    // against 156, 64 x 64 x 64 12.3 against 14.5 (36 shapes of 1-64 rows: 1.14-2.7x).
+    // Not with one or two column tiles of B in rows off 16 bytes and a long K: 16 K
+    // ranges a tile leave most SMs idle, and each copies its B as granules at
+    // latency (us, rows / general: 16 x 33 x 65536 78 / 65, 64 x 1 x 16384 33 / 30, 1
+    // x 129 x 300000 321 / 277; but 64 x 1 x 8192 1.07 x, 16 x 33 x 16384 1.04 x
+    // faster by rows, 255 columns at 32768 1.01-1.1 x).
+    const bool tma = tma_ok(g.B, g.ldb * 4, 1, 0);
+    const bool rows = g.M <= 64 && (tma || g.N >= 224 || g.K <= (g.M > 32 ? 10000 : 20000));
+    if (!cplx && !f16 && ns == 2 && g.batch == 1 && rows && !tune_forced(TUNE_SPLIT_F32)) {
         if (g.M <= 16) return tma ? launch_rows<16, true>(ctx, g, st) : launch_rows<16, false>(ctx, g, st);
         if (g.M <= 32) return tma ? launch_rows<32, true>(ctx, g, st) : launch_rows<32, false>(ctx, g, st);
         return tma ? launch_rows<64, true>(ctx, g, st) : launch_rows<64, false>(ctx, g, st);

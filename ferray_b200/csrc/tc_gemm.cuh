@@ -246,15 +246,16 @@ struct TcSmem {
 // 128-byte row pieces instead of 16 bytes in each of 32 rows (the accumulators
 // come out of TMEM one row per lane).  B200, before and after: i8 8192 x 8192 x 512
 // 117 -> 66 us, 3072^3 33.2 -> 26.4; f16 split 2048^3 99 -> 84; bf16 1024^3 17.1 ->
-// 11.0.  C is read, where it is, the same way.  Up to 32 rows a single warp of the
-// tile stores, and the detour's latency costs more than the pieces save (i8 16 x 1024
-// x 1024 6.7 -> 7.6 us, 32 x 8192 x 8192 20.0 -> 21.0): those rows go straight out.
+// 11.0.  C is read, where it is, the same way.  Up to 64 rows one or two warps of the
+// tile store, and the detour's latency costs more than the pieces save (i8 16 x 1024
+// x 1024 6.7 -> 7.6 us, 33 x 200000 x 128 22.6 -> 28.7, bf16 64 x 50000 x 128 12.4 ->
+// 14.4; over 56 shapes of 33 rows 3-5 %): those rows go straight out.
 template <class Cfg>
 __device__ __forceinline__ void store_block32(const TcArgs& p, int bz, int row0, int gcol0, const uint32_t (&out)[32],
                                               uint4* st) {
     const int lane = threadIdx.x % 32;
     const bool reads = Cfg::EPI == EPI_F32 ? p.beta != 0.f : p.accumulate != 0;
-    if (p.M <= 32 && !reads && gcol0 + 32 <= p.N) {
+    if (p.M <= 64 && !reads && gcol0 + 32 <= p.N) {
         uint32_t* d = static_cast<uint32_t*>(p.C) + bz * p.strideC + (long long)(row0 + lane) * p.ldc + gcol0;
         if (p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(d) & 15) == 0) {
             if (row0 + lane < p.M) {

@@ -339,9 +339,10 @@ static bool packed_pays(int sms, const Gemm& g, TuneChoice table) {
 // at equal split count.
 // `table`: the tuned choice for the shape (its split count fixed when forced).
 // no_room(): what to do without memory for A's copy or the partial products.
+// family: the name it is profiled under (null: the caller's).
 template <class NoRoom>
 static fg_status launch_ffma(fg_ctx* ctx, const Gemm& g, TuneChoice table, int only_tile, cudaStream_t st,
-                             NoRoom no_room) {
+                             NoRoom no_room, const char* family = "ffma_sgemm") {
     const long long M = g.M, N = g.N, K = g.K;
     const long long Mp = (M + 3) / 4 * 4;
     const FfmaChoice c = ffma_plan(ctx->sm_count, M, N, K, g.batch, tune_forced(TUNE_F32) ? table.splits : 0, only_tile,
@@ -360,6 +361,7 @@ static fg_status launch_ffma(fg_ctx* ctx, const Gemm& g, TuneChoice table, int o
         if (splits > 1 && !ws.try_alloc(static_cast<size_t>(splits * M * N * g.batch) * sizeof(float), st))
             return no_room();
     }
+    ProfScope prof(family, st);
     float* At = static_cast<float*>(sa.p);
     transpose_pack_kernel<<<dim3(static_cast<unsigned>((Mp + 63) / 64), static_cast<unsigned>((K + 63) / 64),
                                  static_cast<unsigned>(g.a_count)),
@@ -489,15 +491,11 @@ fg_status launch_simt(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
     }
     const BatchMap bm = batch_map(g);
     if (g.batch > 65535) return set_error(FG_ERR_UNSUPPORTED, "batch above 65535");
-    static const char* names[] = {"simt_dgemm", "simt_sgemm", "simt_zgemm", "simt_cgemm"};
-    const char* fam = g.dtype <= FG_C32 ? names[g.dtype] : "simt";
-    if (g.dtype == FG_F64 || g.dtype == FG_F32) {  // profile under the tuned kernel's name
-        const TuneChoice c = tune_lookup(g.dtype == FG_F64 ? TUNE_F64 : TUNE_F32, g.M, g.N, g.K);
-        if (c.variant == 4 || (g.dtype == FG_F64 && small_dmma(g, c) && !tune_forced(TUNE_F64)))
-            fam = g.dtype == FG_F64 ? "dmma_dgemm" : "ffma_sgemm";
-        else if (c.variant == 5) fam = g.dtype == FG_F64 ? "dmma_dgemm_skinny" : "ffma_sgemm";
-    }
-    ProfScope prof(fam, st);
+    // each launch profiled under the kernel that runs
+    auto named = [st](const char* family, auto launch) {
+        ProfScope prof(family, st);
+        return launch();
+    };
     switch (g.dtype) {
         case FG_F64: {
             const TuneChoice c = tune_lookup(TUNE_F64, g.M, g.N, g.K);
@@ -511,15 +509,18 @@ fg_status launch_simt(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
             // 5.9 against 7.3 us, 128 x 128 x 8 x 100 8.4 against 8.9.  Stacks of few rows and less than two 32 x 256 tiles too
             // (16^3 x 1000 18.6 -> 11.8, 10 x 300 x 300 x 8 18 -> 13; but 8 x 1000 x 1000
             // x 4 24.6 against 28.6).
-            if (!forced && small_dmma(g, c)) return launch_dmma(ctx, g, bm, c.splits, false, st);
-            switch (c.variant) {
-                case 1: return launch_simt_real<double, 4, 4>(g, bm, c.splits, st);
-                case 2: return launch_simt_real<double, 2, 8>(g, bm, c.splits, st);
-                case 3: return launch_simt_real<double, 8, 2>(g, bm, c.splits, st);
-                case 4: return launch_dmma(ctx, g, bm, c.splits, forced, st);
-                case 5: return launch_dmma_skinny(g, bm, c.splits, st);
-                default: return launch_simt_real<double, 8, 8>(g, bm, c.splits, st);
-            }
+            if (c.variant == 4 || (!forced && small_dmma(g, c)))
+                return named("dmma_dgemm", [&] { return launch_dmma(ctx, g, bm, c.splits, forced, st); });
+            if (c.variant == 5)
+                return named("dmma_dgemm_skinny", [&] { return launch_dmma_skinny(g, bm, c.splits, st); });
+            return named("simt_dgemm", [&] {
+                switch (c.variant) {
+                    case 1: return launch_simt_real<double, 4, 4>(g, bm, c.splits, st);
+                    case 2: return launch_simt_real<double, 2, 8>(g, bm, c.splits, st);
+                    case 3: return launch_simt_real<double, 8, 2>(g, bm, c.splits, st);
+                    default: return launch_simt_real<double, 8, 8>(g, bm, c.splits, st);
+                }
+            });
         }
         case FG_F32: {
             const TuneChoice c = tune_lookup(TUNE_F32, g.M, g.N, g.K);
@@ -531,17 +532,19 @@ fg_status launch_simt(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
             // latency (191 x 37 x 44 x 32: 5.9 us, 8.3 with 64).
             if (!forced && g.batch > 1 && (g.M + 63) / 64 * ((g.N + 63) / 64) * g.batch > ctx->sm_count) {
                 const double packed = 4.0 + ffma_plan(ctx->sm_count, g.M, g.N, g.K, g.batch, 0, -1, chain_units(g, c.splits)).us;
-                auto tile64 = [&] { return launch_tile64(g, bm, c, st); };
+                auto tile64 = [&] { return named("sgemm_tile64", [&] { return launch_tile64(g, bm, c, st); }); };
                 if (!ffma_ok(g) || tile64_us(ctx->sm_count, g) < packed) return tile64();
                 return launch_ffma(ctx, g, c, -1, st, tile64);
             }
             auto staged = [&] {
-                switch (c.variant) {
-                    case 1: return launch_simt_real<float, 4, 4>(g, bm, c.splits, st);
-                    case 2: case 5: return launch_simt_real<float, 2, 8>(g, bm, c.splits, st);
-                    case 3: return launch_simt_real<float, 8, 2>(g, bm, c.splits, st);
-                    default: return launch_simt_real<float, 8, 8>(g, bm, c.splits, st);
-                }
+                return named("simt_sgemm", [&] {
+                    switch (c.variant) {
+                        case 1: return launch_simt_real<float, 4, 4>(g, bm, c.splits, st);
+                        case 2: case 5: return launch_simt_real<float, 2, 8>(g, bm, c.splits, st);
+                        case 3: return launch_simt_real<float, 8, 2>(g, bm, c.splits, st);
+                        default: return launch_simt_real<float, 8, 8>(g, bm, c.splits, st);
+                    }
+                });
             };
             if (!forced && c.variant < 4 && g.batch == 1 && ffma_ok(g) && packed_pays(ctx->sm_count, g, c))
                 return launch_ffma(ctx, g, c, -1, st, staged);  // A's copy may not fit: those tiles need none
@@ -549,6 +552,7 @@ fg_status launch_simt(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
             return staged();
         }
         case FG_C64: {
+            ProfScope prof("simt_zgemm", st);
             // Real scalars and one output matrix: the real-embedded GEMM on
             // the DMMA kernel (same 8MNK flops, FP64 FMA per product).
             if (g.batch == 1 && g.alpha_im == 0.0 && g.beta_im == 0.0 && g.K > 0 &&
@@ -578,6 +582,7 @@ fg_status launch_simt(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
             break;
         }
         case FG_C32: {
+            ProfScope prof("simt_cgemm", st);
             // Real scalars, one output matrix and a tuned f32 choice of the
             // cp.async FFMA kernel for the embedded shape: the real-embedded
             // GEMM (M x 2K) (2K x 2N) on it (same 8MNK flops, one FMA per
@@ -599,7 +604,7 @@ fg_status launch_simt(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
                     r.B = bx.p;
                     r.ldb = 2 * g.N;
                     r.ldc = 2 * g.ldc;
-                    return launch_ffma(ctx, r, c, -1, st, ffma_oom);
+                    return launch_ffma(ctx, r, c, -1, st, ffma_oom, nullptr);
                 }
             }
             dim3 grid((g.N + 63) / 64, (g.M + 63) / 64, g.batch);

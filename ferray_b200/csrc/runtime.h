@@ -55,6 +55,7 @@ inline void count_launch(uint64_t n = 1) { g_launches.fetch_add(n, std::memory_o
 
 // Optional per-family kernel timing (fg_profile_enable).  Usage:
 //   ProfScope ps("family", stream); launch<<<...>>>; ps.stop();
+// A null family records nothing.
 extern std::atomic<int> g_prof_on;
 void prof_record(const char* family, cudaEvent_t start, cudaEvent_t stop);
 struct ProfScope {
@@ -62,7 +63,7 @@ struct ProfScope {
     cudaStream_t st;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     ProfScope(const char* family, cudaStream_t stream) : fam(family), st(stream) {
-        if (g_prof_on.load(std::memory_order_relaxed)) {
+        if (family && g_prof_on.load(std::memory_order_relaxed)) {
             cudaEventCreate(&e0);
             cudaEventCreate(&e1);
             cudaEventRecord(e0, st);

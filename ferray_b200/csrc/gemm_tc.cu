@@ -106,10 +106,6 @@ static const char* cfg_name() {
     return "tc_gemm_i8";
 }
 
-static int grid_for_total(long long total) {
-    return static_cast<int>(std::min<long long>(std::max<long long>((total + 255) / 256, 1), 4096));
-}
-
 template <class Cfg>
 static fg_status launch_cfg(fg_ctx* ctx, const TcMaps& maps, TcArgs& args, cudaStream_t st) {
     static std::once_flag once;

@@ -411,14 +411,9 @@ __device__ __forceinline__ void epilogue_store(const TcArgs& p, int bz, int grow
             const uint32_t res = t - __umulhi(t, static_cast<uint32_t>(magic)) * static_cast<uint32_t>(m);
             pk[j / 4] |= res << (8 * (j % 4));
         }
-        if (p.ldc % 16 == 0) {  // whole pieces up to the pitch (planes are 16-byte aligned)
-            *reinterpret_cast<uint4*>(crow) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-            if (gcol0 + 16 < p.ldc) *reinterpret_cast<uint4*>(crow + 16) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-        } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-                if (j < ncols) crow[j] = static_cast<uint8_t>(pk[j / 4] >> (8 * (j % 4)));
-        }
+        // whole pieces up to the pitch (a multiple of 16; planes are 16-byte aligned)
+        *reinterpret_cast<uint4*>(crow) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+        if (gcol0 + 16 < p.ldc) *reinterpret_cast<uint4*>(crow + 16) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
     } else if constexpr (Cfg::EPI == EPI_OZAKI) {
         double* cbase = static_cast<double*>(p.C) + bz * p.strideC;
         // fused groups: weight oz_w 2^(-7d) of group d = oz_d0 - oz_grp (exact)
@@ -488,7 +483,9 @@ __device__ __forceinline__ void epilogue_store(const TcArgs& p, int bz, int grow
                 }
             }
         }
-    } else {  // EPI_F32
+    } else {
+        static_assert(Cfg::EPI == EPI_F32,
+                      "integer outputs leave through shared memory only: fewer stages, to make room for it (epi_staged)");
         float* cbase = static_cast<float*>(p.C) + bz * p.strideC;
         // the FP16 split's operand scaling, undone (exact powers of two)
         const int unscale = p.f16_amax ? -(f16_scale_exp(p.f16_amax[0]) + f16_scale_exp(p.f16_amax[1])) : 0;

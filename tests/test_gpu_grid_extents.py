@@ -12,7 +12,7 @@ def _f32(r, *shape):
     return r.standard_normal(shape, dtype=np.float32)
 
 
-@pytest.mark.parametrize("m,n,k", [(20, 64 * 65536 + 1, 4), (64 * 65536 + 1, 2, 5)])
+@pytest.mark.parametrize("m,n,k", [(32, 64 * 65536 + 1, 16), (64 * 65536 + 1, 2, 5)])
 def test_stack_of_more_tiles_than_a_grid_extent(fg, m, n, k):
     batch = 2
     r = np.random.default_rng(m + n)

@@ -572,6 +572,14 @@ def cpu_baseline(n):
             "sample": "%d of %d rows of C at N=K=%d, %.1f s" % (rows, n, n, dt)}
 
 
+def emit(out, side=None):
+    """The result as one line on stdout, short enough that the last few KB of a log
+    hold all of it; the side measurements (20 KB) as one line on stderr before it."""
+    if side is not None:
+        print(json.dumps({"other_configs": side}), file=sys.stderr, flush=True)
+    print(json.dumps(out), flush=True)
+
+
 def main():
     args = parse()
     if args.peaks:
@@ -803,9 +811,8 @@ def main():
         out["ragged_4096_sharded"] = sharded
     if not args.no_cpu and world == 1:
         out["cpu_baseline"] = cpu_baseline(n)
-    if not args.no_extra and world == 1:
-        out["other_configs"] = side_measurements(fg, L, lib, ctx, stream, n)
-    print(json.dumps(out), flush=True)
+    side = side_measurements(fg, L, lib, ctx, stream, n) if not args.no_extra and world == 1 else None
+    emit(out, side)
     if dist:
         dist.destroy_process_group()
 

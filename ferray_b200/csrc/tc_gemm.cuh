@@ -296,18 +296,42 @@ __device__ __forceinline__ void store_block32(const TcArgs& p, int bz, int row0,
             d += step;
         }
     } else if (vec) {
+        // all reads of C before the stores: one latency a block (i8 4096^3, accumulating,
+        // 83 us with two, 68 with one; 777 x 1001 x 555 quantized, a latency a row, 100
+        // against 55); two where the chunk sums leave fewer registers
+        constexpr int R = Cfg::CHUNKED && Cfg::BN == 256 ? 4 : 8;
 #pragma unroll 1
-        for (int h = 0; h < 2; ++h) {  // 16 rows at a time: all reads of C before the stores
-            uint4 o[4];
+        for (int h = 0; h < 8 / R; ++h) {
+            uint4 o[R];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (16 * h + 4 * i < rows) o[i] = *reinterpret_cast<const uint4*>(d + i * step);
+            for (int i = 0; i < R; ++i)
+                if (4 * (R * h + i) < rows) o[i] = *reinterpret_cast<const uint4*>(d + i * step);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const uint4 v = (i & 1 ? s1 : s0)[128 * h + 32 * i];
-                if (16 * h + 4 * i < rows)
+            for (int i = 0; i < R; ++i) {
+                const uint4 v = (i & 1 ? s1 : s0)[32 * (R * h + i)];
+                if (4 * (R * h + i) < rows)
                     *reinterpret_cast<uint4*>(d) =
                         make_uint4(update(v.x, o[i].x), update(v.y, o[i].y), update(v.z, o[i].z), update(v.w, o[i].w));
+                d += step;
+            }
+        }
+    } else if (reads) {
+        constexpr int R = Cfg::CHUNKED ? 4 : 8;
+#pragma unroll 1
+        for (int h = 0; h < 8 / R; ++h) {
+            uint32_t o[R][4];
+#pragma unroll
+            for (int i = 0; i < R; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (4 * (R * h + i) < rows && col + j < p.N) o[i][j] = d[i * step + j];
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const uint4 v = (i & 1 ? s1 : s0)[32 * (R * h + i)];
+                const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (4 * (R * h + i) < rows && col + j < p.N) d[j] = update(w[j], o[i][j]);
                 d += step;
             }
         }
@@ -318,7 +342,7 @@ __device__ __forceinline__ void store_block32(const TcArgs& p, int bz, int row0,
             const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-                if (col + j < p.N) d[j] = reads ? update(w[j], d[j]) : w[j];
+                if (col + j < p.N) d[j] = w[j];
             d += step;
         }
     }

@@ -72,7 +72,7 @@ struct Tc2Cfg {
 // accumulators are stored one at a time).
 template <class Cfg>
 struct Tc2EpiView {
-    static constexpr int NACC = 1, EPI = Cfg::EPI;
+    static constexpr int NACC = 1, EPI = Cfg::EPI, BN = Cfg::BN, CHUNKED = Cfg::CHUNKED;
 };
 
 template <class Cfg>

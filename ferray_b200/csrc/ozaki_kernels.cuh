@@ -453,8 +453,11 @@ __global__ void __launch_bounds__(256, 4) oz2_residue_b_kernel(
 // Complex: embedded column j < N is Re of column j, j >= N Im of column j - N
 // (interleaved C).  FP64 and instruction issue bound it about evenly (some 70
 // FP64 operations an output at 16 moduli); a thread has four columns, so that one
-// load brings four bytes (two columns: 165 us).  4096^2, 16 moduli: 128 us; 241 with
+// load brings four bytes (two columns: 165 us).  4096^2, 16 moduli: 133 us; 241 with
 // one output a thread, one modulus at a time, base 2^40 and integer carries.
+// Registers: 80 a thread (three blocks an SM) up to 18 moduli, 128 with the fifth
+// digit of 19 and 20 (80: 418 us, 177 so); complex outputs two columns at a time (four
+// at once spill: 4096^2 16 moduli 434 us, 271 so, 19 moduli 1382, 369 so).
 template <int ND>
 __device__ __forceinline__ double oz2_rebuild(double (&d)[ND], const Oz2Consts& c) {
     constexpr double B = 0x1p33, MAGIC = 0x1.8p52;
@@ -470,7 +473,7 @@ __device__ __forceinline__ double oz2_rebuild(double (&d)[ND], const Oz2Consts& 
         d[k] = fma(-cy, B, d[k]);
         d[k + 1] += cy;
     }
-    double t = d[ND - 1];  // |C'| < 2^131: all above digit 2 is exact
+    double t = d[ND - 1];  // |C'| <= K 2^(2P) < 2^135: what lies above digit 2 is an integer below 2^36, exact
 #pragma unroll
     for (int k = ND - 2; k >= 3; --k) t = fma(t, B, d[k]);
     t *= B;
@@ -479,11 +482,11 @@ __device__ __forceinline__ double oz2_rebuild(double (&d)[ND], const Oz2Consts& 
 }
 
 template <int N, bool CPLX>
-__global__ void __launch_bounds__(256, 3) oz2_reconstruct_kernel(
+__global__ void __launch_bounds__(256, N <= 18 ? 3 : 2) oz2_reconstruct_kernel(
     const uint8_t* __restrict__ R, long long M, long long cols, long long pitch, const double* __restrict__ rsc,
     const double* __restrict__ csc, double* __restrict__ C, long long ldc, double alpha, double beta,
     const __grid_constant__ Oz2Consts c) {
-    constexpr int PAIRS = (N + 1) / 2, ND = N <= 18 ? 4 : 5;
+    constexpr int PAIRS = (N + 1) / 2, ND = N <= 18 ? 4 : 5, UNROLL = CPLX ? 2 : 4;
     // complex: even lanes take the real parts of four columns, odd lanes the imaginary
     // ones, and each stores two of the columns
     const int part = CPLX ? threadIdx.x & 1 : 0;
@@ -508,8 +511,8 @@ __global__ void __launch_bounds__(256, 3) oz2_reconstruct_kernel(
             }
         }
         const double rs = ldexp(rsc[i], -2 * c.P) * alpha;
-        double o[4];
-#pragma unroll
+        double o[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll UNROLL
         for (int u = 0; u < 4; ++u) {
             double d[ND];
 #pragma unroll
@@ -522,7 +525,9 @@ __global__ void __launch_bounds__(256, 3) oz2_reconstruct_kernel(
 #pragma unroll
                 for (int k = 0; k < ND; ++k) d[k] = fma(v, c.pW[t][k], d[k]);
             }
-            o[u] = oz2_rebuild<ND>(d, c) * rs * csc[j0 + u < cols ? j0 + u : 0];
+            const double x = oz2_rebuild<ND>(d, c) * rs * csc[j0 + u < cols ? j0 + u : 0];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) o[q] = u == q ? x : o[q];  // no run-time index into registers
         }
         if (CPLX) {
             const double a = __shfl_xor_sync(0xFFFFFFFFu, part ? o[0] : o[2], 1);

@@ -194,10 +194,11 @@ __device__ __forceinline__ void group_range(const TcArgs& p, int gi, int kb0, in
 }
 
 // The groups of work unit t.
+template <class Cfg>
 __device__ __forceinline__ void group_span(const TcArgs& p, int t, int& ga, int& gb) {
     ga = 0;
     gb = max(p.oz_groups, 1);
-    if (p.oz_crt) {
+    if (Cfg::EPI == EPI_CRT) {
         ga = t / (p.batch * p.tiles_m * p.tiles_n);
         gb = ga + 1;
     }
@@ -556,9 +557,9 @@ __device__ __forceinline__ void epilogue_store(const TcArgs& p, int bz, int grow
 template <class Cfg, bool STAGED>
 __device__ __forceinline__ void epilogue_block(const TcArgs& p, const EpiScale& sc, int bz, int row0, int gcol0,
                                                const uint32_t (&v)[Cfg::NACC][32], uint4* st, int oz_grp = 0) {
-    if (row0 >= p.M || gcol0 >= p.N) return;  // the same for the whole warp
     const int grow = row0 + static_cast<int>(threadIdx.x % 32);
     if constexpr (STAGED) {
+        if (row0 >= p.M || gcol0 >= p.N) return;  // the same for the whole warp
         uint32_t out[32];
         epilogue_values<Cfg>(p, sc, grow, gcol0, v, out);
         store_block32<Cfg>(p, bz, row0, gcol0, out, st);
@@ -623,7 +624,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
                 unit_coords(p, t, zo, bz, tm, tn, kb0, kb1);
                 batch_operands(p, bz, za, zb);
                 int ga, gb;
-                group_span(p, t, ga, gb);
+                group_span<Cfg>(p, t, ga, gb);
                 for (int gi = ga; gi < gb && ok; ++gi) {
                 int g0, g1, b_koff;
                 group_range(p, gi, kb0, kb1, g0, g1, b_koff);
@@ -682,7 +683,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
                 int zo, bz, tm, tn, kb0, kb1;
                 unit_coords(p, t, zo, bz, tm, tn, kb0, kb1);
                 int ga, gb;
-                group_span(p, t, ga, gb);
+                group_span<Cfg>(p, t, ga, gb);
                 for (int gi = ga; gi < gb && ok; ++gi) {
                 int g0, g1, b_koff;
                 group_range(p, gi, kb0, kb1, g0, g1, b_koff);
@@ -808,7 +809,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
             bool ok = true;
             for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
                 int ga, gb;
-                group_span(p, t, ga, gb);
+                group_span<Cfg>(p, t, ga, gb);
                 for (int gi = ga; gi < gb; ++gi, ++it) {
                 const int buf = it % Cfg::ACC_BUFS;
                 const uint32_t acc_par = static_cast<uint32_t>((it / Cfg::ACC_BUFS) & 1);

@@ -162,7 +162,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg::THREADS, 1)
                 const int row0 = tm * Cfg::BM + static_cast<int>(rank) * Cfg::CTA_M;
                 const int col0 = tn * Cfg::TILE_N + static_cast<int>(rank) * Cfg::CTA_N;
                 int ga, gb;
-                group_span(p, t, ga, gb);
+                group_span<Cfg>(p, t, ga, gb);
                 for (int gi = ga; gi < gb && ok; ++gi) {
                 int g0, g1, b_koff;
                 group_range(p, gi, kb0, kb1, g0, g1, b_koff);
@@ -225,7 +225,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg::THREADS, 1)
                 int zo, bz, tm, tn, kb0, kb1;
                 unit_coords(p, t, zo, bz, tm, tn, kb0, kb1);
                 int ga, gb;
-                group_span(p, t, ga, gb);
+                group_span<Cfg>(p, t, ga, gb);
                 for (int gi = ga; gi < gb && ok; ++gi) {
                 int g0, g1, b_koff;
                 group_range(p, gi, kb0, kb1, g0, g1, b_koff);
@@ -350,7 +350,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg::THREADS, 1)
                 }
             } else {
                 int ga, gb;
-                group_span(p, t, ga, gb);
+                group_span<Cfg>(p, t, ga, gb);
                 for (int gi = ga; gi < gb; ++gi) {
                 const int buf = it % Cfg::ACC_BUFS;
                 const uint32_t acc_par = static_cast<uint32_t>((it / Cfg::ACC_BUFS) & 1);

@@ -371,9 +371,10 @@ static __global__ void scale_kernel(T* __restrict__ C, long long rows, long long
 // (partials added in split order, round to nearest; beta == 0 leaves C
 // unread), and C[z] = sum (+ C[z] when accumulate) mod 2^32 for int32.  A
 // thread takes V neighbouring outputs of a row (16-byte accesses; the host
-// picks V = 1 where rows break them) and has eight partials in flight: the
-// sums are short, so their latency is what the pass costs (9 splits of 32 x
-// 8192 f32: 6.3 us, 11.4 with one output a thread and one load at a time).
+// picks V = 1 where rows break them or the outputs are few) and has eight partials
+// in flight, 16 with V = 1: the sums are short, so their latency is what the pass
+// costs (9 splits of 32 x 8192 f32: 6.3 us, 11.4 with one output a thread and one load
+// at a time).
 template <typename T, int V>
 static __global__ void __launch_bounds__(256)
     splitk_reduce_kernel(const T* __restrict__ ws, int splits, unsigned M, unsigned N, long long total, T* __restrict__ C,
@@ -381,6 +382,7 @@ static __global__ void __launch_bounds__(256)
     struct alignas(sizeof(T) * V) Vec {
         T x[V];
     };
+    constexpr int U = V == 1 ? 16 : 8;
     const unsigned nv = N / V;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total / V;
          e += (long long)gridDim.x * blockDim.x) {
@@ -391,13 +393,13 @@ static __global__ void __launch_bounds__(256)
         Vec sum;
 #pragma unroll
         for (int j = 0; j < V; ++j) sum.x[j] = T(0);
-        for (int q0 = 0; q0 < splits; q0 += 8) {
-            Vec p[8];
+        for (int q0 = 0; q0 < splits; q0 += U) {
+            Vec p[U];
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
+            for (int u = 0; u < U; ++u)
                 if (q0 + u < splits) p[u] = *reinterpret_cast<const Vec*>(ws + (q0 + u) * total + e * V);
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
+            for (int u = 0; u < U; ++u) {
                 if (q0 + u >= splits) break;
 #pragma unroll
                 for (int j = 0; j < V; ++j) {
@@ -435,7 +437,9 @@ static void splitk_reduce(const T* ws, int splits, long long M, long long N, int
                           long long strideC, T alpha, T beta, int accumulate, cudaStream_t st) {
     constexpr int V = 16 / sizeof(T);
     const long long total = M * N * batch;
-    const bool vec = N % V == 0 && ldc % V == 0 && (batch == 1 || strideC % V == 0) &&
+    // below 32768 outputs fewer, longer threads leave SMs idle (1 x 1000, 64 splits: the
+    // call 47.4 us with 16-byte accesses, 45.3 without)
+    const bool vec = total >= 32768 && N % V == 0 && ldc % V == 0 && (batch == 1 || strideC % V == 0) &&
                      (reinterpret_cast<uintptr_t>(C) & 15) == 0;
     const long long work = vec ? total / V : total;
     const unsigned blocks = static_cast<unsigned>(work < 256 ? 1 : work / 256 < 8192 ? (work + 255) / 256 : 8192);

@@ -107,7 +107,15 @@ static const char* cfg_name() {
 }
 
 template <class Cfg>
+static bool reads_c(const TcArgs& args) {
+    return Cfg::EPI == EPI_F32 ? args.beta != 0.f : args.accumulate != 0;
+}
+
+template <class Cfg>
 static fg_status launch_cfg(fg_ctx* ctx, const TcMaps& maps, TcArgs& args, cudaStream_t st) {
+    if constexpr (TcSmem<Cfg>::STAGED && !Cfg::READS_C) {
+        if (reads_c<Cfg>(args)) return launch_cfg<ReadsC<Cfg>>(ctx, maps, args, st);
+    }
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(once, [] {
@@ -134,6 +142,9 @@ static fg_status launch_cfg(fg_ctx* ctx, const TcMaps& maps, TcArgs& args, cudaS
 // (cudaOccupancyMaxActiveClusters; at most one pair per TPC).
 template <class Cfg>
 static fg_status launch_pair(fg_ctx* ctx, const TcMaps& maps, TcArgs& args, cudaStream_t st) {
+    if constexpr (Tc2Smem<Cfg>::STAGED && !Cfg::READS_C) {
+        if (reads_c<Cfg>(args)) return launch_pair<ReadsC<Cfg>>(ctx, maps, args, st);
+    }
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
     static int max_pairs = 0;
@@ -439,13 +450,16 @@ fg_status launch_qmm(fg_ctx* ctx, long long M, long long N, long long K, const u
 // 119 / 112, 3072^3 55 / 50, 512 x 8192 x 8192 68 / 58 (4 waves against 7 or
 // better); 2560^3 37 / 42, 2304^3 34 / 38, 1536^3 14.3 / 19.5, 2816 x 5632 x 1408
 // 49 / 52 (more).  At 4 against 7 the short runs lose (4096 x 4096 x 1024 39 / 41)
-// and the long ones gain (K >= 2048).  K splits are tuned for the narrow tile.
+// and the long ones gain (K >= 2048), unless C is read, which the wide tile's eight
+// epilogue warps do in two rounds (4096^3 138 / 140).  K splits are tuned for the
+// narrow tile.  (Measured with kernels that could read C too; without, the wide tile
+// is 5-8 % faster: 4096^3 117 -> 108.)
 static bool half_wide(const fg_ctx* ctx, const Gemm& g, int splits) {
     if (splits > 1) return false;
     const long long pairs = ctx->sm_count / 2, rows = (g.M + 255) / 256 * g.batch;
     const long long wide = (rows * ((g.N + 255) / 256) + pairs - 1) / pairs;
     const long long narrow = (rows * ((g.N + 127) / 128) + pairs - 1) / pairs;
-    return 7 * wide < 4 * narrow || (7 * wide == 4 * narrow && g.K >= 2048);
+    return 7 * wide < 4 * narrow || (7 * wide == 4 * narrow && g.K >= 2048 && !g.accumulate);
 }
 
 // bf16 x bf16 / f16 x f16 -> f32 straight from the caller's 16-bit operands

@@ -51,17 +51,18 @@ int* g_sums_dev[kMaxDevices] = {nullptr};
 
 // Once per device, with that device current: the device address of the
 // scratch array (its name in host code is only a host-side stand-in) and
-// the kernel's shared-memory opt-in.
+// the two kernels' shared-memory opt-in.
 fg_status setup_device(int device, int** out) {
     std::lock_guard<std::mutex> lk(g_setup_mu);
     if (g_sums_dev[device] == nullptr) {
         void* p = nullptr;
         cudaError_t e = cudaGetSymbolAddress(&p, g_qmm_sums);
         if (e != cudaSuccess) return fgrt::cuda_error(e, "cudaGetSymbolAddress(qmm scratch)");
-        e = cudaFuncSetAttribute(fg::tc_gemm_kernel<CfgQmmNoAlloc>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(fg::tc_smem_bytes<CfgQmmNoAlloc>()));
-        if (e != cudaSuccess) return fgrt::cuda_error(e, "cudaFuncSetAttribute(qmm no-alloc)");
+        for (auto kernel : {fg::tc_gemm_kernel<CfgQmmNoAlloc>, fg::tc_gemm_kernel<fg::ReadsC<CfgQmmNoAlloc>>}) {
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     static_cast<int>(fg::tc_smem_bytes<CfgQmmNoAlloc>()));
+            if (e != cudaSuccess) return fgrt::cuda_error(e, "cudaFuncSetAttribute(qmm no-alloc)");
+        }
         g_sums_dev[device] = static_cast<int*>(p);
     }
     *out = g_sums_dev[device];
@@ -151,7 +152,8 @@ extern "C" fg_status fg_quantized_matmul_noalloc(fg_ctx* ctx, size_t m, size_t n
     args.timeout_ns = 4000000000ull;
     const long long tiles = (long long)args.tiles_m * args.tiles_n;
     const int grid = static_cast<int>(std::min<long long>(tiles, ctx->sm_count));
-    fg::tc_gemm_kernel<CfgQmmNoAlloc><<<grid, CfgQmmNoAlloc::THREADS, fg::tc_smem_bytes<CfgQmmNoAlloc>(), st>>>(maps, args);
+    auto kernel = accumulate ? fg::tc_gemm_kernel<fg::ReadsC<CfgQmmNoAlloc>> : fg::tc_gemm_kernel<CfgQmmNoAlloc>;
+    kernel<<<grid, CfgQmmNoAlloc::THREADS, fg::tc_smem_bytes<CfgQmmNoAlloc>(), st>>>(maps, args);
     count_launch();
     FG_CUDA(cudaGetLastError());
     return FG_OK;

@@ -69,9 +69,20 @@ struct TcCfg {
     static constexpr int ACC_BUFS = (4 * ACC_COLS <= 512) ? 4 : (2 * ACC_COLS <= 512) ? 2 : 1;
     static constexpr int TMEM_COLS = 512;
     static constexpr int THREADS = 192;
+    static constexpr bool READS_C = false;  // see ReadsC
     static_assert(ACC_COLS <= 512, "accumulators exceed TMEM");
     static_assert(BN % 16 == 0 && BN <= 256, "UMMA N");
     static_assert(BN % B_CHUNK_ELEMS == 0, "B tile must be whole 128-byte chunks");
+};
+
+// A configuration with staged stores whose products read C (beta, accumulate), as a
+// kernel of its own: the reads of a block before its stores take registers and code
+// that the others do without (one kernel for both: bf16 2048 x 2048 x 512 14.4 us,
+// 1024^3 12.2; apart 12.4 and 10.4, and the 256 x 256 tile's spills go from 572 bytes
+// to 96).
+template <class Cfg>
+struct ReadsC : Cfg {
+    static constexpr bool READS_C = true;
 };
 
 struct TcMaps {
@@ -255,7 +266,7 @@ template <class Cfg>
 __device__ __forceinline__ void store_block32(const TcArgs& p, int bz, int row0, int gcol0, const uint32_t (&out)[32],
                                               uint4* st) {
     const int lane = threadIdx.x % 32;
-    const bool reads = Cfg::EPI == EPI_F32 ? p.beta != 0.f : p.accumulate != 0;
+    constexpr bool reads = Cfg::READS_C;
     if (p.M <= 64 && !reads && gcol0 + 32 <= p.N) {
         uint32_t* d = static_cast<uint32_t*>(p.C) + bz * p.strideC + (long long)(row0 + lane) * p.ldc + gcol0;
         if (p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(d) & 15) == 0) {

@@ -62,6 +62,7 @@ struct Tc2Cfg {
     static constexpr int EPI_WARPS = CHUNKED && BN == 256 ? 8 : 4;
     static constexpr int EPI_COLS = BN * 4 / EPI_WARPS;  // columns per epilogue warp
     static constexpr int THREADS = 64 + 32 * EPI_WARPS;
+    static constexpr bool READS_C = false;  // see ReadsC
     static_assert(ACC_COLS <= 512, "accumulators exceed TMEM");
     static_assert(BN % 32 == 0 && BN <= 256, "UMMA N (pair)");
     static_assert(CTA_N % B_CHUNK_ELEMS == 0, "B half must be whole 128-byte chunks");
@@ -73,6 +74,7 @@ struct Tc2Cfg {
 template <class Cfg>
 struct Tc2EpiView {
     static constexpr int NACC = 1, EPI = Cfg::EPI, BN = Cfg::BN, CHUNKED = Cfg::CHUNKED;
+    static constexpr bool READS_C = Cfg::READS_C;
 };
 
 template <class Cfg>

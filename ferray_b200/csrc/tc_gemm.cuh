@@ -260,14 +260,16 @@ struct TcSmem {
 // 117 -> 66 us, 3072^3 33.2 -> 26.4; f16 split 2048^3 99 -> 84; bf16 1024^3 17.1 ->
 // 11.0.  C is read, where it is, the same way.  Up to 64 rows one or two warps of the
 // tile store, and the detour's latency costs more than the pieces save (i8 16 x 1024
-// x 1024 6.7 -> 7.6 us, 33 x 200000 x 128 22.6 -> 28.7, bf16 64 x 50000 x 128 12.4 ->
-// 14.4; over 56 shapes of 33 rows 3-5 %): those rows go straight out.
+// x 1024 6.7 -> 7.6 us, 33 x 10000 x 256 6.2 -> 8.2, bf16 64 x 50000 x 128 12.4 ->
+// 14.4; over 40 shapes of 33 rows 6-14 %): those rows go straight out, unless N is so
+// long that a CTA stores tile after tile and the pieces count again, and then
+// only up to 32 (i8 64 x 200000 x 64 40 straight, 33 staged).
 template <class Cfg>
 __device__ __forceinline__ void store_block32(const TcArgs& p, int bz, int row0, int gcol0, const uint32_t (&out)[32],
                                               uint4* st) {
     const int lane = threadIdx.x % 32;
     constexpr bool reads = Cfg::READS_C;
-    if (p.M <= 64 && !reads && gcol0 + 32 <= p.N) {
+    if (p.M <= (p.N <= 65536 ? 64 : 32) && !reads && gcol0 + 32 <= p.N) {
         uint32_t* d = static_cast<uint32_t*>(p.C) + bz * p.strideC + (long long)(row0 + lane) * p.ldc + gcol0;
         if (p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(d) & 15) == 0) {
             if (row0 + lane < p.M) {

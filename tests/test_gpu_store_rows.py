@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("off,pad", [(0, 0), (0, 4), (0, 3), (1, 0)])
-@pytest.mark.parametrize("m,n", [(33, 64), (48, 300), (63, 256), (64, 100), (64, 257), (65, 96)])
+@pytest.mark.parametrize("m,n", [(33, 64), (48, 300), (63, 256), (64, 100), (64, 257), (65, 96), (33, 65600)])
 @pytest.mark.parametrize("dtype", ["i8", "i16", "bf16"])
 def test_store_rows(fg, dtype, m, n, off, pad):
     from ferray_b200 import _lib as L

@@ -372,17 +372,17 @@ static __global__ void scale_kernel(T* __restrict__ C, long long rows, long long
 // unread), and C[z] = sum (+ C[z] when accumulate) mod 2^32 for int32.  A
 // thread takes V neighbouring outputs of a row (16-byte accesses; the host
 // picks V = 1 where rows break them or the outputs are few) and has eight partials
-// in flight, 16 with V = 1: the sums are short, so their latency is what the pass
-// costs (9 splits of 32 x 8192 f32: 6.3 us, 11.4 with one output a thread and one load
-// at a time).
-template <typename T, int V>
+// in flight, 16 where they are few (elsewhere 16 are slower: 777 x 1001 in rows off 16
+// bytes, the call 61 against 55 us): the sums are short, so their latency is what the
+// pass costs (9 splits of 32 x 8192 f32: 6.3 us, 11.4 with one output a thread and one
+// load at a time).
+template <typename T, int V, int U>
 static __global__ void __launch_bounds__(256)
     splitk_reduce_kernel(const T* __restrict__ ws, int splits, unsigned M, unsigned N, long long total, T* __restrict__ C,
                          long long ldc, long long strideC, T alpha, T beta, int accumulate) {
     struct alignas(sizeof(T) * V) Vec {
         T x[V];
     };
-    constexpr int U = V == 1 ? 16 : 8;
     const unsigned nv = N / V;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total / V;
          e += (long long)gridDim.x * blockDim.x) {
@@ -439,16 +439,14 @@ static void splitk_reduce(const T* ws, int splits, long long M, long long N, int
     const long long total = M * N * batch;
     // below 32768 outputs fewer, longer threads leave SMs idle (1 x 1000, 64 splits: the
     // call 47.4 us with 16-byte accesses, 45.3 without)
-    const bool vec = total >= 32768 && N % V == 0 && ldc % V == 0 && (batch == 1 || strideC % V == 0) &&
+    const bool few = total < 32768;
+    const bool vec = !few && N % V == 0 && ldc % V == 0 && (batch == 1 || strideC % V == 0) &&
                      (reinterpret_cast<uintptr_t>(C) & 15) == 0;
     const long long work = vec ? total / V : total;
     const unsigned blocks = static_cast<unsigned>(work < 256 ? 1 : work / 256 < 8192 ? (work + 255) / 256 : 8192);
-    if (vec)
-        splitk_reduce_kernel<T, V><<<blocks, 256, 0, st>>>(ws, splits, static_cast<unsigned>(M), static_cast<unsigned>(N),
-                                                           total, C, ldc, strideC, alpha, beta, accumulate);
-    else
-        splitk_reduce_kernel<T, 1><<<blocks, 256, 0, st>>>(ws, splits, static_cast<unsigned>(M), static_cast<unsigned>(N),
-                                                           total, C, ldc, strideC, alpha, beta, accumulate);
+    auto kernel = few ? splitk_reduce_kernel<T, 1, 16> : vec ? splitk_reduce_kernel<T, V, 8> : splitk_reduce_kernel<T, 1, 8>;
+    kernel<<<blocks, 256, 0, st>>>(ws, splits, static_cast<unsigned>(M), static_cast<unsigned>(N), total, C, ldc, strideC,
+                                   alpha, beta, accumulate);
 }
 
 }  // namespace fg

@@ -12,7 +12,9 @@
 // alignment works).  Warps form a 2 x 2 grid of 32 x 32 or 64 x 32 warp tiles of
 // 8 x 8 MMAs.  The DMMA pipe bounds it; one CTA of 256 threads and 128 x 128 an SM
 // waited at its barrier (2048^3 670 us), two or three small ones fill each other's
-// waits (560 us, 30.7 TFLOP/s).  FOLD: accumulation runs of `seg` K blocks, each
+// waits (560 us, 30.7 TFLOP/s).  Few rows take a 32 x 256 tile of 256 threads, two CTAs
+// an SM as well (with one, 158 registers a thread: 32 x 8192 x 8192 211 us, 188 with
+// two; 3000 x 3000 x 64 72, 62).  FOLD: accumulation runs of `seg` K blocks, each
 // added to the sum of the earlier ones, so that a CTA with all of K rounds like the
 // split-K form with one run a CTA.
 // Fragments (m8n8k4, f64): A row = lane / 4, col = lane % 4; B row =
@@ -39,7 +41,7 @@ struct DmmaTile {
     static constexpr int WARPS_M = WARPS_M_, WARPS_N = WARPS_N_, MT = MT_;
     static constexpr int BM = WARPS_M * MT * 8, BN = WARPS_N * 32, BK = FG_DMMA_BK, STAGES = 3;
     static constexpr int THREADS = 32 * WARPS_M * WARPS_N;
-    static constexpr int MIN_CTAS = THREADS == 256 ? 1 : BM * BN <= 64 * 64 ? 3 : 2;
+    static constexpr int MIN_CTAS = BM * BN <= 64 * 64 ? 3 : 2;  // an SM
     static constexpr int APAD = 4, BPAD = 4;
     static constexpr int A_ELEMS = BM * (BK + APAD);
     static constexpr int B_ELEMS = BK * (BN + BPAD);
@@ -96,7 +98,8 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MIN_CTAS)
     const int m0 = blockIdx.y * Cfg::BM, n0 = blockIdx.x * Cfg::BN;
     const int kblocks = (K + Cfg::BK - 1) / Cfg::BK;
 
-    // global -> shared: BM*BK/256 A and BK*BN/256 B elements per thread per stage
+    // global -> shared, per thread and stage: BM * BK / W / THREADS copies of A, BK * BN / W /
+    // THREADS of B
     auto load_stage = [&](int stage, int kb) {
         const int k0 = kb * Cfg::BK;
         double* as = As + stage * Cfg::A_ELEMS;

@@ -479,8 +479,15 @@ static fg_status launch_gemv(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
 }
 
 // A plain DGEMM that leaves the table's variant for the small DMMA tiles.
-static bool small_dmma(const Gemm& g, const TuneChoice& c) {
+static bool small_dmma(int sms, const Gemm& g, const TuneChoice& c) {
     if (c.variant == 5) return g.batch > 1 && g.N < 512;
+    if (c.variant == 1 && g.batch > 1 && g.K <= 24) {
+        // two short K blocks: not where the last wave of 64 x 64 tiles, three an SM, is
+        // mostly empty (40 x 300 x 300 x 16 16.5 us register-staged, 18.5 so; 100 x 128 x
+        // 128 x 24 12.3, 10.3 so)
+        const long long units = (g.M + 63) / 64 * ((g.N + 63) / 64) * g.batch, slots = 3LL * sms;
+        if (5 * units < 4 * ((units + slots - 1) / slots) * slots) return false;
+    }
     return c.variant < 4 && g.K > (g.batch > 1 ? 8 : 16);
 }
 
@@ -509,7 +516,7 @@ fg_status launch_simt(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
             // 5.9 against 7.3 us, 128 x 128 x 8 x 100 8.4 against 8.9.  Stacks of few rows and less than two 32 x 256 tiles too
             // (16^3 x 1000 18.6 -> 11.8, 10 x 300 x 300 x 8 18 -> 13; but 8 x 1000 x 1000
             // x 4 24.6 against 28.6).
-            if (c.variant == 4 || (!forced && small_dmma(g, c)))
+            if (c.variant == 4 || (!forced && small_dmma(ctx->sm_count, g, c)))
                 return named("dmma_dgemm", [&] { return launch_dmma(ctx, g, bm, c.splits, forced, st); });
             if (c.variant == 5)
                 return named("dmma_dgemm_skinny", [&] { return launch_dmma_skinny(g, bm, c.splits, st); });
@@ -528,9 +535,11 @@ fg_status launch_simt(fg_ctx* ctx, const Gemm& g, cudaStream_t st) {
             // Stacks: one CTA of 64 threads per tile or the packed kernel,
             // whichever its model puts first (96 x 80 x 64 x 512: 22 us against 33,
             // 47 register-staged; 300 x 700 x 2000 x 3: 135 against 70), unless there
-            // are fewer tiles than SMs, where 256 threads a tile have the shorter
-            // latency (191 x 37 x 44 x 32: 5.9 us, 8.3 with 64).
-            if (!forced && g.batch > 1 && (g.M + 63) / 64 * ((g.N + 63) / 64) * g.batch > ctx->sm_count) {
+            // are fewer tiles than SMs, or with a K of one or two blocks than twice
+            // the SMs, where 256 threads a tile have the shorter latency (191 x 37 x 44 x
+            // 32: 5.9 us, 8.3 with 64; 826 x 157 x 17 x 6 6.2, 8.2).
+            const long long stack_tiles = (g.M + 63) / 64 * ((g.N + 63) / 64) * g.batch;
+            if (!forced && g.batch > 1 && stack_tiles > (g.K <= 24 ? 2 : 1) * ctx->sm_count) {
                 const double packed = 4.0 + ffma_plan(ctx->sm_count, g.M, g.N, g.K, g.batch, 0, -1, chain_units(g, c.splits)).us;
                 auto tile64 = [&] { return named("sgemm_tile64", [&] { return launch_tile64(g, bm, c, st); }); };
                 if (!ffma_ok(g) || tile64_us(ctx->sm_count, g) < packed) return tile64();

@@ -70,6 +70,7 @@ struct fgrt::GroupedJob {
     std::vector<Opnd> oa, ob;
     std::vector<Zero> zeros;
     long long total_tiles = 0;
+    int edge = 64;  // plain FP32: rows and columns of a tile
     long long arena = 0;
     int nseg = 0;
     int njobs = 0;  // prep launch blocks: segments cut at PREP_JOB_CHUNKS chunks
@@ -133,7 +134,16 @@ fg_status grouped_job_build(fg_ctx* ctx, fg_dtype dtype, fg_mode mode, const fg_
     // longest K first: the static strided tile walk then balances SMs
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return table[x].k > table[y].k; });
     const int np = static_cast<int>(order.size());
-    const int bm = j->kind == 0 ? 64 : 128;
+    int bm = 128;
+    if (j->kind == 0) {
+        // 32 x 32 tiles where they all run at once (six CTAs an SM): a 64 x 64 tile is
+        // two warps, too few alone on an SM (us, 128-thread tiles of before / 64 x 64 /
+        // 32 x 32: 5 problems of 64 x 64 x 2000 112 / 131 / 56, 148 of them 124 / 135 /
+        // 105, 50 of 100 x 100 x 1000 86 / 80 / 72; 250 of 64 x 64 x 64 13.2 / 10.6 / 12.7).
+        long long whole = 0;
+        for (int x : order) whole += (table[x].m + 63) / 64 * ((table[x].n + 63) / 64);
+        bm = j->edge = 2 * whole <= 3LL * ctx->sm_count ? 32 : 64;
+    }
     j->probs_in.resize(np);
     j->probs.resize(np);
     j->oa.resize(np);
@@ -252,7 +262,8 @@ fg_status grouped_job_bind(GroupedJob* j, void* dev_base, void* host_stage) {
                     const int x = order[i];
                     const GroupedProblem& g = j->probs[x];
                     // rows / columns of tiles with both halves
-                    const int fm = std::min((g.M + 31) / 64, g.tiles_m), fn = std::min((g.N + 31) / 64, g.tiles_n);
+                    const int fm = j->edge == 32 ? 0 : std::min((g.M + 31) / 64, g.tiles_m);
+                    const int fn = j->edge == 32 ? 0 : std::min((g.N + 31) / 64, g.tiles_n);
                     for (int tm = type & 2 ? fm : 0; tm < (type & 2 ? g.tiles_m : fm); ++tm)
                         for (int tn = type & 1 ? fn : 0; tn < (type & 1 ? g.tiles_n : fn); ++tn)
                             htiles[t++] = TileRec{x, tm, tn, g.k_blocks};
@@ -387,7 +398,8 @@ static fg_status grouped_job_kernels(GroupedJob* j, cudaStream_t st) {
     FG_CUDA(cudaMemsetAsync(j->d_counter, 0, sizeof(unsigned long long), st));
     if (j->kind == 0) {
         ProfScope prof("simt_grouped_sgemm", st);
-        simt_grouped_sgemm<<<std::min<long long>(j->total_tiles, ctx->sm_count * 6), 64, 0, st>>>(j->sargs);
+        auto kernel = j->edge == 32 ? simt_grouped_sgemm<32> : simt_grouped_sgemm<64>;
+        kernel<<<std::min<long long>(j->total_tiles, ctx->sm_count * 6), 64, 0, st>>>(j->sargs);
         prof.stop();
     } else if (j->kind == 1) {
         ProfScope prof("tc_grouped_i8", st);

@@ -589,8 +589,8 @@ static __global__ void __launch_bounds__(256) grouped_prep_kernel(const PrepSeg*
 }
 
 // ------------------------------------------------------------------ SIMT
-// Plain FP32 grouped GEMM: CTAs of 64 threads walk the batch's 64 x 64 tiles
-// (ffma_tile64.cuh), handed out by an atomic counter, longest K first.  4096
+// Plain FP32 grouped GEMM: CTAs of 64 threads walk the batch's 64 x 64 (few: 32 x 32)
+// tiles (ffma_tile64.cuh), handed out by an atomic counter, longest K first.  4096
 // problems with dims log-uniform in [8, 512] (14.4 GFLOP useful, 18.3 padded to
 // 32) take 485 us a call on a B200, against 769 with 128-thread tiles of scalar
 // FMAs padded to 64 (or 32 with 2 x 4 outputs a thread); 338 such problems 81
@@ -613,6 +613,8 @@ struct SimtGroupedArgs {
     float alpha, beta;
 };
 
+// EDGE: rows and columns of a tile, 64 or 32.
+template <int EDGE>
 static __global__ void __launch_bounds__(64, 6) simt_grouped_sgemm(const SimtGroupedArgs g) {
     __shared__ Tile64Smem s;
     // The first tile of a CTA is its block index; the next one is claimed before
@@ -626,9 +628,9 @@ static __global__ void __launch_bounds__(64, 6) simt_grouped_sgemm(const SimtGro
     long long t = 0;
     for (;;) {
         const SimtProblem r = g.problems[tr.problem];
-        const int m0 = tr.tm * 64, n0 = tr.tn * 64;
+        const int m0 = tr.tm * EDGE, n0 = tr.tn * EDGE;
         sgemm_tile64<false, false>(
-            Tile64Args{min(r.m - m0, 64), min(r.n - n0, 64), r.k, r.a + m0 * r.lda, r.b + n0, r.c + m0 * r.ldc + n0, r.lda,
+            Tile64Args{min(r.m - m0, EDGE), min(r.n - n0, EDGE), r.k, r.a + m0 * r.lda, r.b + n0, r.c + m0 * r.ldc + n0, r.lda,
                        r.ldb, r.ldc, g.alpha, g.beta},
             0, 0, s,
             [&] {

@@ -264,12 +264,15 @@ struct TcSmem {
 // 14.4; over 40 shapes of 33 rows 6-14 %): those rows go straight out, unless N is so
 // long that a CTA stores tile after tile and the pieces count again, and then
 // only up to 32 (i8 64 x 200000 x 64 40 straight, 33 staged).
-template <class Cfg>
+__device__ __forceinline__ bool few_rows(const TcArgs& p) { return p.M <= (p.N <= 65536 ? 64 : 32); }
+
+// FEW: the rows that go straight out are stored here too.
+template <class Cfg, bool FEW = true>
 __device__ __forceinline__ void store_block32(const TcArgs& p, int bz, int row0, int gcol0, const uint32_t (&out)[32],
                                               uint4* st) {
     const int lane = threadIdx.x % 32;
     constexpr bool reads = Cfg::READS_C;
-    if (p.M <= (p.N <= 65536 ? 64 : 32) && !reads && gcol0 + 32 <= p.N) {
+    if (FEW && !reads && few_rows(p) && gcol0 + 32 <= p.N) {
         uint32_t* d = static_cast<uint32_t*>(p.C) + bz * p.strideC + (long long)(row0 + lane) * p.ldc + gcol0;
         if (p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(d) & 15) == 0) {
             if (row0 + lane < p.M) {
@@ -567,7 +570,7 @@ __device__ __forceinline__ void epilogue_store(const TcArgs& p, int bz, int grow
 
 // A warp's 32 x 32 block of the tile, lane i holding row row0 + i; st: the
 // warp's staging memory (unused by the row-wise epilogues).
-template <class Cfg, bool STAGED>
+template <class Cfg, bool STAGED, bool FEW = true>
 __device__ __forceinline__ void epilogue_block(const TcArgs& p, const EpiScale& sc, int bz, int row0, int gcol0,
                                                const uint32_t (&v)[Cfg::NACC][32], uint4* st, int oz_grp = 0) {
     const int grow = row0 + static_cast<int>(threadIdx.x % 32);
@@ -575,7 +578,7 @@ __device__ __forceinline__ void epilogue_block(const TcArgs& p, const EpiScale& 
         if (row0 >= p.M || gcol0 >= p.N) return;  // the same for the whole warp
         uint32_t out[32];
         epilogue_values<Cfg>(p, sc, grow, gcol0, v, out);
-        store_block32<Cfg>(p, bz, row0, gcol0, out, st);
+        store_block32<Cfg, FEW>(p, bz, row0, gcol0, out, st);
     } else {
         epilogue_store<Cfg>(p, bz, grow, gcol0, v, oz_grp);
     }
@@ -836,16 +839,42 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
                 const int row0 = tm * Cfg::BM + ew * 32;
                 const uint32_t row_addr = tmem + (static_cast<uint32_t>(ew * 32) << 16) + buf * Cfg::ACC_COLS;
                 if constexpr (Cfg::NACC == 1 && STAGED) {
-                    uint32_t v[2][1][32];  // the next block in flight behind the stores of this one
-                    tmem_ld_32x32b_x32(row_addr, v[0][0]);
+                    const int col0 = tn * Cfg::BN, blocks = row0 < p.M ? min(Cfg::BN / 32, (p.N - col0 + 31) / 32) : 0;
+                    int c = 0;
+                    if constexpr (!Cfg::READS_C) {
+                        // Few rows: whole blocks straight out, in a loop of its own: these
+                        // calls are short, and fetching the staged store's code costs them
+                        // more than it does (i8 16 x 4000 x 256 7.6 us by it, 6.2 so).
+                        const int grow = row0 + lane;
+                        uint32_t* d = static_cast<uint32_t*>(p.C) + zo * p.strideC + (long long)grow * p.ldc + col0;
+                        if (few_rows(p) && p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(d) & 15) == 0) {
 #pragma unroll 1
-                    for (int c = 0; c < Cfg::BN / 32; c += 2) {
+                            for (; c < blocks && col0 + 32 * c + 32 <= p.N; ++c) {
+                                uint32_t v[1][32], out[32];
+                                tmem_ld_32x32b_x32(row_addr + c * 32, v[0]);
+                                tmem_wait_ld(v[0]);
+                                epilogue_values<Cfg>(p, sc, grow, col0 + 32 * c, v, out);
+                                if (grow < p.M) {
+#pragma unroll
+                                    for (int j = 0; j < 32; j += 4)
+                                        *reinterpret_cast<uint4*>(d + 32 * c + j) =
+                                            make_uint4(out[j], out[j + 1], out[j + 2], out[j + 3]);
+                                }
+                            }
+                        }
+                    }
+                    uint32_t v[2][1][32];  // the next block in flight behind the stores of this one
+                    if (c < blocks) tmem_ld_32x32b_x32(row_addr + c * 32, v[0][0]);
+#pragma unroll 1
+                    for (; c < blocks; c += 2) {
 #pragma unroll
                         for (int h = 0; h < 2; ++h) {
-                            tmem_wait_ld(v[h][0]);
-                            if (c + h + 1 < Cfg::BN / 32) tmem_ld_32x32b_x32(row_addr + (c + h + 1) * 32, v[h ^ 1][0]);
-                            epilogue_block<Cfg, STAGED>(p, sc, zo, row0, tn * Cfg::BN + (c + h) * 32, v[h],
-                                                        s.epi[STAGED ? ew : 0], gi);
+                            if (c + h < blocks) {
+                                tmem_wait_ld(v[h][0]);
+                                if (c + h + 1 < blocks) tmem_ld_32x32b_x32(row_addr + (c + h + 1) * 32, v[h ^ 1][0]);
+                                epilogue_block<Cfg, STAGED, false>(p, sc, zo, row0, col0 + (c + h) * 32, v[h],
+                                                                   s.epi[STAGED ? ew : 0], gi);
+                            }
                         }
                     }
                 } else {

@@ -371,11 +371,11 @@ static __global__ void scale_kernel(T* __restrict__ C, long long rows, long long
 // (partials added in split order, round to nearest; beta == 0 leaves C
 // unread), and C[z] = sum (+ C[z] when accumulate) mod 2^32 for int32.  A
 // thread takes V neighbouring outputs of a row (16-byte accesses; the host
-// picks V = 1 where rows break them or the outputs are few) and has eight partials
-// in flight, 16 where they are few (elsewhere 16 are slower: 777 x 1001 in rows off 16
-// bytes, the call 61 against 55 us): the sums are short, so their latency is what the
-// pass costs (9 splits of 32 x 8192 f32: 6.3 us, 11.4 with one output a thread and one
-// load at a time).
+// picks V = 1 where rows break them or few outputs have many splits) and has eight
+// partials in flight, 16 in the last case (elsewhere 16 are slower: 777 x 1001 in rows
+// off 16 bytes, the call 61 against 55 us, 2 x 20 of 9 splits 14.4 against 13.4): the sums
+// are short, so their latency is what the pass costs (9 splits of 32 x 8192 f32: 6.3 us,
+// 11.4 with one output a thread and one load at a time).
 template <typename T, int V, int U>
 static __global__ void __launch_bounds__(256)
     splitk_reduce_kernel(const T* __restrict__ ws, int splits, unsigned M, unsigned N, long long total, T* __restrict__ C,
@@ -437,9 +437,9 @@ static void splitk_reduce(const T* ws, int splits, long long M, long long N, int
                           long long strideC, T alpha, T beta, int accumulate, cudaStream_t st) {
     constexpr int V = 16 / sizeof(T);
     const long long total = M * N * batch;
-    // below 32768 outputs fewer, longer threads leave SMs idle (1 x 1000, 64 splits: the
-    // call 47.4 us with 16-byte accesses, 45.3 without)
-    const bool few = total < 32768;
+    // below 32768 outputs of many splits fewer, longer threads leave SMs idle (1 x 1000,
+    // 64 splits: the call 47.4 us with 16-byte accesses, 45.3 without)
+    const bool few = total < 32768 && splits > 16;
     const bool vec = !few && N % V == 0 && ldc % V == 0 && (batch == 1 || strideC % V == 0) &&
                      (reinterpret_cast<uintptr_t>(C) & 15) == 0;
     const long long work = vec ? total / V : total;

@@ -320,14 +320,15 @@ static bool rows16(const void* X, long long ld, long long count, long long mstri
 //    copy of A is most of the work: 33 x 7000 x 1100 41 / 26, 3000 x 64 x 2000 37 /
 //    28, but 7000 x 9 x 3000 81 / 101, 1000 x 64 x 2000 21 / 23;
 //  * with few outputs where K is long and B comes in whole granules: 300 x 100 x
-//    6000 39 / 33, 64 x 20 x 12000 47 / 37, but 300 x 33 x 6000 28 / 31;
+//    6000 39 / 33, 64 x 20 x 12000 47 / 37, 2 x 20 x 3000 18.5 / 16.5, but 300 x 33 x 6000
+//    28 / 31;
 //  * few rows of a wide B: 17 x 1000 x 3000 1.18 x;
 //  * where the table's 64 x 64 tiles times its splits just pass one wave: 220 x 130
 //    x 3365 29 / 25 (220 x 65 x 3365 22 / 25).
 static bool packed_pays(int sms, const Gemm& g, TuneChoice table) {
     if (g.K <= 1024) return false;
     if (g.N > 32 && g.M * g.N >= 90000) return true;
-    if (g.K >= 6000 && g.M <= 1000 && rows16(g.B, g.ldb, 1, 0)) return true;
+    if (g.K >= (g.M <= 32 ? 3000 : 6000) && g.M <= 1000 && rows16(g.B, g.ldb, 1, 0)) return true;
     if (table.variant == 2 && g.N >= 1000) return true;
     int kps = 0;
     const int splits = plan_splits(table.splits, static_cast<int>((g.K + 63) / 64), g.M * g.N, sizeof(float), &kps);
@@ -424,13 +425,13 @@ static fg_status launch_tile64(const Gemm& g, const BatchMap& bm, TuneChoice tab
                        static_cast<float*>(g.C), g.lda, g.ldb, g.ldc, (float)g.alpha_re, (float)g.beta_re};
     const int chain = 4 * chain_units(g, table.splits);  // 16-deep K blocks
     const bool vec = rows16(g.A, g.lda, g.a_count, g.a_mstride) && rows16(g.B, g.ldb, g.b_count, g.b_mstride);
-    const long long tiles = tm * tn, gy = std::min<long long>(tiles, 65535), gz = (tiles + gy - 1) / gy;
-    if (tiles > 0x7FFF0000ll) return set_error(FG_ERR_UNSUPPORTED, "stacked matrix above 2^31 tiles");
+    const bool tall = tm > tn;
+    const long long longer = std::max(tm, tn), gy = std::min<long long>(longer, 65535), chunks = (longer + gy - 1) / gy;
+    const long long gz = std::min(tm, tn) * chunks;
+    if (gz > 65535) return set_error(FG_ERR_UNSUPPORTED, "stacked matrix of too many tiles");
     const dim3 grid(static_cast<unsigned>(g.batch), static_cast<unsigned>(gy), static_cast<unsigned>(gz));
-    if (vec)
-        sgemm_tile64_kernel<true><<<grid, 64, 0, st>>>(a, bm, static_cast<int>(tn), static_cast<int>(tiles), chain);
-    else
-        sgemm_tile64_kernel<false><<<grid, 64, 0, st>>>(a, bm, static_cast<int>(tn), static_cast<int>(tiles), chain);
+    auto kernel = vec ? sgemm_tile64_kernel<true> : sgemm_tile64_kernel<false>;
+    kernel<<<grid, 64, 0, st>>>(a, bm, tall, static_cast<int>(longer), static_cast<int>(chunks), chain);
     count_launch();
     FG_CUDA(cudaGetLastError());
     return FG_OK;

@@ -354,20 +354,25 @@ static fg_status launch_ffma(fg_ctx* ctx, const Gemm& g, TuneChoice table, int o
     if ((long long)splits * g.batch > 65535) return set_error(FG_ERR_UNSUPPORTED, "batch above 65535");
     Scratch sa, ws;
     if (!sa.try_alloc(static_cast<size_t>(g.a_count * K * Mp) * sizeof(float), st)) return no_room();
-    if (splits > 1 && !ws.try_alloc(static_cast<size_t>(splits * M * N * g.batch) * sizeof(float), st)) {
-        // the table's own split count keeps the length of an accumulation run too
-        const int fewer = plan_splits(table.splits, kunits, M * N * g.batch, sizeof(float), &kps);
-        if (fewer >= splits) return no_room();
-        splits = fewer;
-        if (splits > 1 && !ws.try_alloc(static_cast<size_t>(splits * M * N * g.batch) * sizeof(float), st))
-            return no_room();
-    }
+    // before the next allocation, which the device then does not wait for (32 x 8192 x 8192:
+    // the call 119 us, 121 after it)
     ProfScope prof(family, st);
     float* At = static_cast<float*>(sa.p);
     transpose_pack_kernel<<<dim3(static_cast<unsigned>((Mp + 63) / 64), static_cast<unsigned>((K + 63) / 64),
                                  static_cast<unsigned>(g.a_count)),
                             256, 0, st>>>(static_cast<const float*>(g.A), (int)M, (int)K, g.lda, g.a_mstride, At, Mp);
     count_launch();
+    if (splits > 1 && !ws.try_alloc(static_cast<size_t>(splits * M * N * g.batch) * sizeof(float), st)) {
+        // the table's own split count keeps the length of an accumulation run too
+        const int fewer = plan_splits(table.splits, kunits, M * N * g.batch, sizeof(float), &kps);
+        const bool room = fewer < splits &&
+                          (fewer == 1 || ws.try_alloc(static_cast<size_t>(fewer * M * N * g.batch) * sizeof(float), st));
+        if (!room) {
+            prof.drop();
+            return no_room();
+        }
+        splits = fewer;
+    }
     BatchMap bm = batch_map(g);
     for (int d = 0; d < 4; ++d) bm.a_bstride[d] = g.a_istride[d] * K * Mp;
     float* C = static_cast<float*>(g.C);

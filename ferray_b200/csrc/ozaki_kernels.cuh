@@ -313,8 +313,9 @@ __device__ __forceinline__ uint2 oz2_biased(double v) {
 
 // Symmetric residues in [-(m/2), m - 1 - (m/2)] of eight such integers, packed.
 // The integer's bytes times 256^b mod m (two dp4a) give an x < 2^20 of the same
-// residue, x mod m is the high word of (x ceil(2^32 / m) mod 2^32) m, and m/2,
-// added before, is taken off all four bytes of a word at once.
+// residue, x mod m is the high word of (x ceil(2^32 / m) mod 2^32) m (Lemire, Kaser
+// and Kurz, "Faster remainder by direct computation", 2019), and m/2, added before, is
+// taken off all four bytes of a word at once.
 __device__ __forceinline__ uint2 oz2_pack8(const uint2 (&a)[8], const Oz2Consts& c, int l) {
     const uint32_t m = static_cast<uint32_t>(c.m[l]), magic = c.magic[l], c_lo = c.c_lo[l], c_hi = c.c_hi[l];
     const uint32_t corr = c.corr[l], h4 = (m / 2) * 0x01010101u;
@@ -447,7 +448,8 @@ __global__ void __launch_bounds__(256, 4) oz2_residue_b_kernel(
 // add up to less than 2^20); q = rint(sum / Mp) (at most n, far from a tie),
 // the digits of C' follow exactly and are balanced into [-2^32, 2^32] with exact
 // carries.  The digits above the two lowest are joined first, what that rounds off
-// is added to the lowest, and the final sum is the one rounding that counts
+// (Dekker's Fast2Sum) is added to the lowest, and the final sum is the one rounding that
+// counts
 // (rounding twice showed: 17 moduli 1.3e-18 of ||A|| ||B|| at 2048^3, 2e-19 so).
 // Then C = alpha 2^(e_i + f_j - 2P) C' (+ beta C).
 // Complex: embedded column j < N is Re of column j, j >= N Im of column j - N

@@ -76,6 +76,13 @@ struct ProfScope {
             e0 = e1 = nullptr;
         }
     }
+    void drop() {  // record nothing after all
+        if (e0) {
+            cudaEventDestroy(e0);
+            cudaEventDestroy(e1);
+            e0 = e1 = nullptr;
+        }
+    }
     ~ProfScope() { stop(); }
 };
 
